@@ -205,7 +205,7 @@ StepArgs<T> make_args(const vi_plan *p, const vi_medium *m, const vi_fields *f) 
   const vi_config &c = p->cfg;
   StepArgs<T> a;
   std::memset(&a, 0, sizeof(a));
-  a.nx = c.nx;
+  a.nx = a.ld = a.ldz = c.nx;
   a.nz = c.nz;
   a.nsls = c.nsls;
   a.Lx = p->Lx;
@@ -370,6 +370,20 @@ template int launch_finite_check<float>(const void *, const void *, const void *
 template int launch_finite_check<double>(const void *, const void *, const void *, long long, int *, int,
                                          cudaStream_t);
 
+// Grids of more than one tile of the fused kernel (64 x 32 cells) whose rows
+// or planes the split kernels cannot take as they are run the split pair on
+// padded copies (split.cu:padded_split_steps); a grid within one tile keeps
+// the fused kernel, one launch of one CTA per step.  Measured on B200, us per
+// step of a 64-step call, copies included, against the fused kernel: 47 x 45
+// ISO FP32 9.6 vs 33.5, 301 x 203 10.5 vs 35.8, 1001 x 501 VTI 18.6 vs 44.5
+// (FP64 38.7 vs 102, TTI 23.7 vs 52.8), 1403 x 597 VTI 24.6 vs 57.2; of a
+// 1-step call 1001 x 501 137 vs 196 (both then copy the whole state), 47 x 45
+// 59 vs 91.  The line is not a crossover (no size was found where the fused
+// kernel wins): tiny grids keep the path callers see reported for them.  The
+// choice depends on the grid alone, so steps divided over calls give the same
+// bits.
+constexpr long long kPadMinCells = 2048;
+
 template <typename T>
 static int step_impl(vi_plan *p, const vi_medium *m, vi_fields *f, const vi_shot *s, int it0,
                      int nsteps, int variant, cudaStream_t st) {
@@ -448,9 +462,15 @@ static int step_impl(vi_plan *p, const vi_medium *m, vi_fields *f, const vi_shot
     if (rc) return rc;
     p->last_kernel = variant == 0 ? 5 : variant;
   } else {
-    rc = fused_steps<T>(p, a, s, it0, nsteps, st, variant);
+    rc = VI_ERR_BUDGET;
+    if (variant == 0 && (long long)p->cfg.nx * p->cfg.nz >= kPadMinCells)
+      rc = padded_split_steps<T>(p, a, s, it0, nsteps, st);
+    p->last_kernel = 5;
+    if (rc == VI_ERR_BUDGET) {  // small grids, or no memory for the padded planes
+      rc = fused_steps<T>(p, a, s, it0, nsteps, st, variant);
+      p->last_kernel = p->last_used_tma ? (variant == 4 ? 4 : 3) : 2;
+    }
     if (rc) return rc;
-    p->last_kernel = p->last_used_tma ? (variant == 4 ? 4 : 3) : 2;
   }
   if (variant == 1) p->last_kernel = 1;
   // paths without the folded finite check get it once at the end of the call
@@ -557,7 +577,7 @@ extern "C" int vi_plan_destroy(vi_plan *p) {
   cudaGetDevice(&prev);
   cudaSetDevice(p->device);
   void *bufs[] = {p->psix, p->psiz, p->tabx, p->tabz, p->scratch, p->alt, p->slo,
-                  p->dsrc, p->damp, p->drec, p->tile_lists, p->fwd, p->errflag, p->wave_ctl};
+                  p->dsrc, p->damp, p->drec, p->tile_lists, p->fwd, p->errflag, p->wave_ctl, p->pad};
   for (void *b : bufs)
     if (b) cudaFree(b);
   cudaSetDevice(prev);

@@ -37,6 +37,9 @@ constexpr double kD8[4] = {1225.0 / 1024.0, -245.0 / 3072.0, 49.0 / 5120.0,
 template <typename T>
 struct StepArgs {
   int nx, nz, nsls;
+  int ld;               // row stride of the state and medium planes: nx, or (split kernels) nx
+                        // rounded up to a multiple of 4 in planes laid out by the plan
+  int ldz;              // row stride of the z strips' psi planes
   int Lx, Rx, Tz, Bz;   // CPML strip widths (cells) per side
   int wx, hz;           // wx = Lx + Rx, hz = Tz + Bz
   T dt;

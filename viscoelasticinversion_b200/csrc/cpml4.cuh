@@ -6,7 +6,7 @@
 // plan's tables and its memory in psi plane Pn.  psi is read from `in` and,
 // when `store`, written to `out` (the same set in place, the other set for
 // the ping-pong forms).  A group whose four cells lie in one x strip with
-// 16-byte aligned memory runs as 4-wide loads and stores; any other group
+// 16-byte aligned memory (psi and, by nx % 4 == 0, the profile rows) runs as 4-wide loads and stores; any other group
 // cell by cell; both round the same way (cpml_mem / cpml_rate), so the
 // results do not depend on the form.
 #pragma once
@@ -29,7 +29,7 @@ __device__ __forceinline__ void cpml_x4(const StepArgs<T> &args, int gi0, int gj
   const long long pl = args.psix_plane;
   const int xs0 = strip_x(gi0, nx, args.Lx, args.Rx);
   const long long o0 = (long long)gj * args.wx + xs0;
-  if (xs0 >= 0 && strip_x(gi0 + 3, nx, args.Lx, args.Rx) == xs0 + 3 && ((o0 | pl) & 3) == 0) {
+  if (xs0 >= 0 && strip_x(gi0 + 3, nx, args.Lx, args.Rx) == xs0 + 3 && ((o0 | pl | nx) & 3) == 0) {
     const Q4<T> q0 = ldc4(in + r0.p * pl + o0), q1 = ldc4(in + r1.p * pl + o0);
     const Q4<T> B0 = ldg4(tb + r0.b * nx + gi0), A0 = ldg4(tb + r0.a * nx + gi0), K0 = ldg4(tb + r0.k * nx + gi0);
     const Q4<T> B1 = ldg4(tb + r1.b * nx + gi0), A1 = ldg4(tb + r1.a * nx + gi0), K1 = ldg4(tb + r1.k * nx + gi0);
@@ -70,10 +70,10 @@ __device__ __forceinline__ void cpml_x4(const StepArgs<T> &args, int gi0, int gj
 template <typename T>
 __device__ __forceinline__ void cpml_z4(const StepArgs<T> &args, int zs, int gi0, int gj, CpmlRows r0, CpmlRows r1,
                                         const T *in, T *out, bool store, Q4<T> &d0, Q4<T> &d1) {
-  const int nx = args.nx, nz = args.nz;
+  const int nz = args.nz;
   const T *tb = args.tz;
   const long long pl = args.psiz_plane;
-  const long long o = (long long)zs * nx + gi0;
+  const long long o = (long long)zs * args.ldz + gi0;
   const T B0 = tb[r0.b * nz + gj], A0 = tb[r0.a * nz + gj], K0 = tb[r0.k * nz + gj];
   const T B1 = tb[r1.b * nz + gj], A1 = tb[r1.a * nz + gj], K1 = tb[r1.k * nz + gj];
   Q4<T> q0, q1, p0, p1;

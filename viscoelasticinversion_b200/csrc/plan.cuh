@@ -23,6 +23,10 @@ struct vi_plan {
   void *tabx = nullptr, *tabz = nullptr;  // 6*nx and 6*nz reals
   void *scratch = nullptr;                // plain path: 6 planes
   void *alt = nullptr;                    // fused path: second v/sigma copy (5 planes)
+  // split step on grids whose rows need padding: state, medium, TTI's
+  // second memory-variable set (grown on demand)
+  void *pad = nullptr;
+  size_t pad_bytes = 0;
   // VI_F32C split step: the stresses' rounding residues (3 bfloat16
   // planes), part of the plan's state like the CPML memory; slo_valid is
   // false after a step that did not carry them (they restart from zero)

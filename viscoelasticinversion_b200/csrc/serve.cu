@@ -131,6 +131,9 @@ int64_t footprint(const vi_request &r) {
   const int64_t tr = 2 * (int64_t)r.nrec * r.nt * e;
   const int64_t wav = (int64_t)r.nsrc * (r.wavelet_nt > 0 ? r.wavelet_nt : 0) * e;
   int64_t b = (8 + 2 * ns + 6) * np * e + psi + 2 * tr + wav + (16 << 20);
+  // odd rows: the padded copies hold the state and the medium (within the
+  // planes above for ISO and VTI) and TTI's second memory-variable set
+  if (c.nx % 4 != 0 && c.medium == VI_MEDIUM_TTI) b += (2 + 3 * (int64_t)c.nsls) * np * e;
   if (r.kind == VI_REQ_GRADIENT) {
     int64_t K = 1;
     while (K * K < r.nt) ++K;

@@ -62,19 +62,19 @@ namespace vb {
 
 
 // AFDA: the grid has the H-AFDA free surface (a separate instantiation,
-// so the others carry none of its code)
-template <typename T, bool PP, bool HINT, bool AFDA>
+// so the others carry none of its code); RAG: nx % 4 != 0
+template <typename T, bool PP, bool HINT, bool AFDA, bool RAG>
 __global__ void __launch_bounds__(SplitVelTma<T>::NT, (sizeof(T) == 4 ? 1024 : 512) / SplitVelTma<T>::NT)
     k_split_vel_tma(const __grid_constant__ StepArgs<T> a, const FusedExtras<T> x, const __grid_constant__ SplitMaps maps) {
-  split_vel_tma_tile<T, PP, HINT, AFDA>(a, x, maps, blockIdx.x);
+  split_vel_tma_tile<T, PP, HINT, AFDA, RAG>(a, x, maps, blockIdx.x);
   split_vel_sample<T>(a, x, blockIdx.x);
 }
 
-template <typename T, bool PP, bool OOP, bool HINT, bool AFDA>
+template <typename T, bool PP, bool OOP, bool HINT, bool AFDA, bool RAG>
 __global__ void __launch_bounds__(SplitGeom<T>::NT, (sizeof(T) == 4 ? 1024 : 512) / SplitGeom<T>::NT)
     k_split_vel_ldg(const __grid_constant__ StepArgs<T> a, const FusedExtras<T> x) {
   pdl_wait();  // the previous stress pass is complete and visible
-  split_vel_tile<T, PP, OOP, HINT, AFDA>(a, x, blockIdx.x);
+  split_vel_tile<T, PP, OOP, HINT, AFDA, RAG>(a, x, blockIdx.x);
   split_vel_sample<T, OOP>(a, x, blockIdx.x);
 }
 
@@ -163,23 +163,24 @@ static int launch_stress(const StepArgs<T> &a, const FusedExtras<T> &x, const Sp
                   : launch_stress_k<T, KIND, NSLS, false, false>(a, x, m, ntiles, st, pdl);
 }
 
-template <typename T, bool AFDA>
+template <typename T, bool AFDA, bool RAG>
 static cudaError_t launch_vel_ldg_k(const StepArgs<T> &a, const FusedExtras<T> &x, int ntiles, cudaStream_t st,
                                     bool pdl) {
   using G = SplitGeom<T>;
   const bool oop = a.vx_o != nullptr, pp = oop || a.psix_o != a.psix || a.psiz_o != a.psiz;
-  return oop        ? launch_pdl(k_split_vel_ldg<T, true, true, true, AFDA>, dim3(ntiles), dim3(G::NT), 0, st, pdl, a, x)
-         : pp       ? (x.l2hint ? launch_pdl(k_split_vel_ldg<T, true, false, true, AFDA>, dim3(ntiles), dim3(G::NT), 0, st, pdl, a, x)
-                                : launch_pdl(k_split_vel_ldg<T, true, false, false, AFDA>, dim3(ntiles), dim3(G::NT), 0, st, pdl, a, x))
-         : x.l2hint ? launch_pdl(k_split_vel_ldg<T, false, false, true, AFDA>, dim3(ntiles), dim3(G::NT), 0, st, pdl, a, x)
-                    : launch_pdl(k_split_vel_ldg<T, false, false, false, AFDA>, dim3(ntiles), dim3(G::NT), 0, st, pdl, a, x);
+  return oop        ? launch_pdl(k_split_vel_ldg<T, true, true, true, AFDA, RAG>, dim3(ntiles), dim3(G::NT), 0, st, pdl, a, x)
+         : pp       ? (x.l2hint ? launch_pdl(k_split_vel_ldg<T, true, false, true, AFDA, RAG>, dim3(ntiles), dim3(G::NT), 0, st, pdl, a, x)
+                                : launch_pdl(k_split_vel_ldg<T, true, false, false, AFDA, RAG>, dim3(ntiles), dim3(G::NT), 0, st, pdl, a, x))
+         : x.l2hint ? launch_pdl(k_split_vel_ldg<T, false, false, true, AFDA, RAG>, dim3(ntiles), dim3(G::NT), 0, st, pdl, a, x)
+                    : launch_pdl(k_split_vel_ldg<T, false, false, false, AFDA, RAG>, dim3(ntiles), dim3(G::NT), 0, st, pdl, a, x);
 }
 
 template <typename T>
 int launch_split_vel(const StepArgs<T> &a, const FusedExtras<T> &x, int ntiles, cudaStream_t st,
                      bool pdl) {
-  const cudaError_t e = x.fs == kFsAfda ? launch_vel_ldg_k<T, true>(a, x, ntiles, st, pdl)
-                                        : launch_vel_ldg_k<T, false>(a, x, ntiles, st, pdl);
+  const cudaError_t e = x.fs == kFsAfda ? launch_vel_ldg_k<T, true, false>(a, x, ntiles, st, pdl)
+                        : a.nx % 4 != 0 ? launch_vel_ldg_k<T, false, true>(a, x, ntiles, st, pdl)
+                                        : launch_vel_ldg_k<T, false, false>(a, x, ntiles, st, pdl);
   return cuda_check(e, "split velocity launch");
 }
 
@@ -268,7 +269,7 @@ bool split_eligible(const vi_plan *p, const StepArgs<T> &a) {
   return true;
 }
 
-template <typename T, bool AFDA>
+template <typename T, bool AFDA, bool RAG>
 static int launch_vel_tma_k(const StepArgs<T> &a, const FusedExtras<T> &x, const SplitMaps &m,
                             int ntiles, cudaStream_t st, bool pdl) {
   using G = SplitVelTma<T>;
@@ -277,43 +278,42 @@ static int launch_vel_tma_k(const StepArgs<T> &a, const FusedExtras<T> &x, const
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(attr_set & (1ULL << dev))) {
-    for (auto k : {k_split_vel_tma<T, true, true, AFDA>, k_split_vel_tma<T, false, true, AFDA>,
-                   k_split_vel_tma<T, true, false, AFDA>, k_split_vel_tma<T, false, false, AFDA>}) {
+    for (auto k : {k_split_vel_tma<T, true, true, AFDA, RAG>, k_split_vel_tma<T, false, true, AFDA, RAG>,
+                   k_split_vel_tma<T, true, false, AFDA, RAG>, k_split_vel_tma<T, false, false, AFDA, RAG>}) {
       const cudaError_t ea = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
       if (ea != cudaSuccess) return cuda_check(ea, "split velocity (TMA) smem attribute");
     }
     attr_set |= 1ULL << dev;
   }
   const cudaError_t e =
-      pp ? (x.l2hint ? launch_pdl(k_split_vel_tma<T, true, true, AFDA>, dim3(ntiles), dim3(G::NT), (size_t)G::SMEM, st, pdl, a, x, m)
-                     : launch_pdl(k_split_vel_tma<T, true, false, AFDA>, dim3(ntiles), dim3(G::NT), (size_t)G::SMEM, st, pdl, a, x, m))
-         : (x.l2hint ? launch_pdl(k_split_vel_tma<T, false, true, AFDA>, dim3(ntiles), dim3(G::NT), (size_t)G::SMEM, st, pdl, a, x, m)
-                     : launch_pdl(k_split_vel_tma<T, false, false, AFDA>, dim3(ntiles), dim3(G::NT), (size_t)G::SMEM, st, pdl, a, x, m));
+      pp ? (x.l2hint ? launch_pdl(k_split_vel_tma<T, true, true, AFDA, RAG>, dim3(ntiles), dim3(G::NT), (size_t)G::SMEM, st, pdl, a, x, m)
+                     : launch_pdl(k_split_vel_tma<T, true, false, AFDA, RAG>, dim3(ntiles), dim3(G::NT), (size_t)G::SMEM, st, pdl, a, x, m))
+         : (x.l2hint ? launch_pdl(k_split_vel_tma<T, false, true, AFDA, RAG>, dim3(ntiles), dim3(G::NT), (size_t)G::SMEM, st, pdl, a, x, m)
+                     : launch_pdl(k_split_vel_tma<T, false, false, AFDA, RAG>, dim3(ntiles), dim3(G::NT), (size_t)G::SMEM, st, pdl, a, x, m));
   return cuda_check(e, "split velocity (TMA) launch");
 }
 
 template <typename T>
 static int launch_vel_tma(const StepArgs<T> &a, const FusedExtras<T> &x, const SplitMaps &m,
                           int ntiles, cudaStream_t st, bool pdl) {
-  return x.fs == kFsAfda ? launch_vel_tma_k<T, true>(a, x, m, ntiles, st, pdl)
-                         : launch_vel_tma_k<T, false>(a, x, m, ntiles, st, pdl);
+  // planes padded by the plan have an imaging surface or none
+  return x.fs == kFsAfda ? launch_vel_tma_k<T, true, false>(a, x, m, ntiles, st, pdl)
+         : a.nx % 4 != 0 ? launch_vel_tma_k<T, false, true>(a, x, m, ntiles, st, pdl)
+                         : launch_vel_tma_k<T, false, false>(a, x, m, ntiles, st, pdl);
 }
 
+// The time loop on planes of row stride a.ld (16-byte aligned, a.ld % 4 ==
+// 0).  pad_m: the second memory-variable set of a TTI run on planes laid out
+// by the plan (plane stride a.ld * nz), else in p->alt; *m_last, if given,
+// receives where the memory variables end, else they are copied back to a.m.
 template <typename T>
-int split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st,
-                int mode) {
+static int split_run(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st, int mode,
+                     T *pad_m = nullptr, T **m_last = nullptr) {
   const bool pipelined = mode == kSplitPipelined, vel_tma = mode == kSplitVelTma;
   using G = SplitGeom<T>;
   const vi_config &c = p->cfg;
   const bool tti = c.medium == VI_MEDIUM_TTI;
-  if (!split_eligible<T>(p, a))
-    return set_error(VI_ERR_ARG, "split step needs nx % 4 == 0 and 16-byte aligned planes");
-  if (pipelined && tti)
-    return set_error(VI_ERR_ARG, "the pipelined split step covers ISO and VTI media");
-  if (pipelined && !split_p_fits(c.medium, c.nsls, (int)sizeof(T)))
-    return set_error(VI_ERR_ARG, "pipelined split step does not fit shared memory for this medium");
-  if (nsteps == 0) return VI_OK;
-  const size_t np = (size_t)c.nx * c.nz;
+  const size_t np = (size_t)a.ld * c.nz;
   int rc = VI_OK;
   if constexpr (sizeof(T) == 4) {
     if (c.precision == VI_F32C) {
@@ -338,7 +338,7 @@ int split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps
   const long long user_ms = a.mstride;
   if (tti && c.nsls > 0) {
     // the plan's second state copy holds the other memory-variable set
-    if (!p->alt) {
+    if (!pad_m && !p->alt) {
       const size_t bytes = (5 + 3 * (size_t)c.nsls) * np * sizeof(T);
       size_t have = 0;
       rc = ensure_buffer(p, &p->alt, &have, bytes);
@@ -346,7 +346,7 @@ int split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps
       rc = cuda_check(cudaMemsetAsync(p->alt, 0, bytes, st), "zero alt state");
       if (rc) return rc;
     }
-    alt_m = (T *)p->alt + 5 * np;
+    alt_m = pad_m ? pad_m : (T *)p->alt + 5 * np;
   }
   // per-tile source/receiver lists of the velocity tiling and (pipelined:
   // its own 64 x 8 tiling) the stress tiling, in one buffer
@@ -380,14 +380,14 @@ int split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps
   } else {
     const int bw = tti ? SplitTtiGeom<T>::BW : SplitStressGeom<T>::BW;
     const int bh = tti ? SplitTtiGeom<T>::BH : SplitStressGeom<T>::BH;
-    if ((rc = encode_map(&ms.a, a.vx, e, c.nx, c.nz, 1, 0, bw, bh, 1))) return rc;
-    if ((rc = encode_map(&ms.b, a.vz, e, c.nx, c.nz, 1, 0, bw, bh, 1))) return rc;
+    if ((rc = encode_map(&ms.a, a.vx, e, a.ld, c.nz, 1, 0, bw, bh, 1))) return rc;
+    if ((rc = encode_map(&ms.b, a.vz, e, a.ld, c.nz, 1, 0, bw, bh, 1))) return rc;
     ms.c = ms.b;
     if (vel_tma) {
       using VG = SplitVelTma<T>;
-      if ((rc = encode_map(&mv.a, a.sxx, e, c.nx, c.nz, 1, 0, VG::WX, VG::TZ, 1))) return rc;
-      if ((rc = encode_map(&mv.b, a.sxz, e, c.nx, c.nz, 1, 0, VG::WX, VG::HZ, 1))) return rc;
-      if ((rc = encode_map(&mv.c, a.szz, e, c.nx, c.nz, 1, 0, VG::WZ, VG::HZ, 1))) return rc;
+      if ((rc = encode_map(&mv.a, a.sxx, e, a.ld, c.nz, 1, 0, VG::WX, VG::TZ, 1))) return rc;
+      if ((rc = encode_map(&mv.b, a.sxz, e, a.ld, c.nz, 1, 0, VG::WX, VG::HZ, 1))) return rc;
+      if ((rc = encode_map(&mv.c, a.szz, e, a.ld, c.nz, 1, 0, VG::WZ, VG::HZ, 1))) return rc;
     }
   }
   FusedExtras<T> x;
@@ -450,7 +450,9 @@ int split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps
       if ((rc = launch_split_stress<T>(c.medium, a, xs, ms, sntiles, st, true))) return rc;
     }
   }
-  if (alt_m && nsteps % 2 == 1) {
+  if (m_last) {
+    *m_last = alt_m && nsteps % 2 == 1 ? alt_m : user_m;
+  } else if (alt_m && nsteps % 2 == 1) {
     // the memory variables sit in the plan's copy: bring them back
     for (int q = 0; q < 3 * c.nsls; ++q) {
       rc = cuda_check(cudaMemcpyAsync(user_m + q * user_ms, alt_m + q * np, np * sizeof(T),
@@ -462,12 +464,114 @@ int split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps
   return VI_OK;
 }
 
+template <typename T>
+int split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st,
+                int mode) {
+  const bool pipelined = mode == kSplitPipelined;
+  const vi_config &c = p->cfg;
+  if (!split_eligible<T>(p, a))
+    return set_error(VI_ERR_ARG, "split step needs nx % 4 == 0 and 16-byte aligned planes");
+  if (pipelined && c.medium == VI_MEDIUM_TTI)
+    return set_error(VI_ERR_ARG, "the pipelined split step covers ISO and VTI media");
+  if (pipelined && !split_p_fits(c.medium, c.nsls, (int)sizeof(T)))
+    return set_error(VI_ERR_ARG, "pipelined split step does not fit shared memory for this medium");
+  if (nsteps == 0) return VI_OK;
+  return split_run<T>(p, a, s, it0, nsteps, st, mode);
+}
+
+// ---- grids whose rows the split kernels cannot take as they are ----------
+
+// Copies planes between row strides: columns [c0, c1), rows from r0 (planes
+// 2 .. 4: from r0s) to r1.  One plane per blockIdx.z, 8 rows x 128 columns
+// per block.  Bandwidth bound: each value read and written once.
+template <typename T>
+struct PadPlanes {
+  const T *src[5 + 3 * VI_MAX_SLS + 8];
+  T *dst[5 + 3 * VI_MAX_SLS + 8];
+};
+template <typename T>
+__global__ void __launch_bounds__(256) k_copy_planes(const __grid_constant__ PadPlanes<T> pl, int lds, int ldd, int c0,
+                                                     int c1, int r0, int r0s, int r1) {
+  const int q = blockIdx.z, j = blockIdx.y * 8 + threadIdx.x / 32;
+  if (j < (q >= 2 && q < 5 ? r0s : r0) || j >= r1) return;
+  const T *src = pl.src[q] + (long long)j * lds;
+  T *dst = pl.dst[q] + (long long)j * ldd;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int i = c0 + (int)blockIdx.x * 128 + 32 * k + (int)(threadIdx.x % 32);
+    if (i < c1) dst[i] = src[i];
+  }
+}
+
+// The split pair for rows that are no multiple of 4 cells, or planes off a
+// 16-byte boundary: state and medium are copied once per call into planes of
+// the plan whose rows start on 16-byte boundaries, stepped there, and the
+// updated cells of the state copied back.  Groups that reach past the update
+// region keep their outer cells (keep_edge4).
+template <typename T>
+int padded_split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st) {
+  const vi_config &c = p->cfg;
+  if (nsteps == 0) return VI_OK;
+  const int nx = c.nx, nz = c.nz, ld = (nx + 3) / 4 * 4, ns = 5 + 3 * c.nsls;
+  const size_t np = (size_t)ld * nz;
+  const T *med[8] = {a.rho, a.c11, a.c13, a.c15, a.c33, a.c35, a.c55, a.tau};
+  int nmed = 0;
+  for (const T *m : med) nmed += m != nullptr;
+  const bool tti = c.medium == VI_MEDIUM_TTI;
+  const size_t need = (ns + nmed + (tti ? 3 * c.nsls : 0)) * np * sizeof(T);
+  int rc;
+  if (p->pad_bytes < need) {
+    if ((rc = ensure_buffer(p, &p->pad, &p->pad_bytes, need))) return rc;
+    if ((rc = cuda_check(cudaMemsetAsync(p->pad, 0, need, st), "zero padded planes"))) return rc;
+  }
+  T *base = (T *)p->pad;
+  PadPlanes<T> pl;
+  T *user[5] = {a.vx, a.vz, a.sxx, a.szz, a.sxz};
+  for (int q = 0; q < ns; ++q) {
+    pl.src[q] = q < 5 ? user[q] : a.m + (q - 5) * a.mstride;
+    pl.dst[q] = base + q * np;
+  }
+  const T **slot[8] = {&a.rho, &a.c11, &a.c13, &a.c15, &a.c33, &a.c35, &a.c55, &a.tau};
+  int q = ns;
+  for (int k = 0; k < 8; ++k)
+    if (med[k]) {
+      pl.src[q] = med[k];
+      *slot[k] = pl.dst[q] = base + q * np;
+      ++q;
+    }
+  T *const user_m = a.m;
+  const long long user_ms = a.mstride;
+  k_copy_planes<T><<<dim3((nx + 127) / 128, (nz + 7) / 8, q), 256, 0, st>>>(pl, nx, ld, 0, nx, 0, 0, nz);
+  if ((rc = cuda_check(cudaGetLastError(), "pad launch"))) return rc;
+  a.ld = ld;
+  a.vx = base;
+  a.vz = base + np;
+  a.sxx = base + 2 * np;
+  a.szz = base + 3 * np;
+  a.sxz = base + 4 * np;
+  a.m = base + 5 * np;
+  a.mstride = (long long)np;
+  T *m_last = nullptr;
+  if ((rc = split_run<T>(p, a, s, it0, nsteps, st, kSplitVelTma, tti ? base + (ns + nmed) * np : nullptr, &m_last)))
+    return rc;
+  for (int k = 0; k < ns; ++k) {
+    pl.src[k] = k < 5 ? base + k * np : m_last + (k - 5) * np;
+    pl.dst[k] = k < 5 ? user[k] : user_m + (k - 5) * user_ms;
+  }
+  k_copy_planes<T><<<dim3((nx - 2 * L + 127) / 128, (nz + 7) / 8, ns), 256, 0, st>>>(pl, ld, nx, L, nx - L, L, 0,
+                                                                                     nz - L);
+  return cuda_check(cudaGetLastError(), "unpad launch");
+}
+
 template bool split_eligible<float>(const vi_plan *, const StepArgs<float> &);
 template bool split_eligible<double>(const vi_plan *, const StepArgs<double> &);
 template int split_steps<float>(vi_plan *, StepArgs<float>, const vi_shot *, int, int, cudaStream_t,
                                 int);
 template int split_steps<double>(vi_plan *, StepArgs<double>, const vi_shot *, int, int,
                                  cudaStream_t, int);
+
+template int padded_split_steps<float>(vi_plan *, StepArgs<float>, const vi_shot *, int, int, cudaStream_t);
+template int padded_split_steps<double>(vi_plan *, StepArgs<double>, const vi_shot *, int, int, cudaStream_t);
 
 template int launch_split_vel_batch<float>(int, bool, const BatchDev<float> &, int, int, cudaStream_t, bool);
 template int launch_split_vel_batch<double>(int, bool, const BatchDev<double> &, int, int, cudaStream_t,

@@ -131,6 +131,11 @@ template <typename T>
 int split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st,
                 int mode);
 
+// The same steps for rows and planes the split kernels cannot take as they
+// are (nx % 4 != 0, unaligned planes), on copies laid out by the plan.
+template <typename T>
+int padded_split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st);
+
 // The time-blocked form of the split pair (wave.cu): one persistent
 // kernel runs sweeps of k steps as a wavefront over 8-row bands, with a
 // lag of d bands between consecutive passes (plan's wave_k / wave_d, 0 =

@@ -27,8 +27,10 @@ namespace vb {
 // 4-cell group whose stress derivatives' raw parts are in hxx/hxz (row
 // windows) and zxz/zzz (z derivatives).
 // OOP: the new velocities go to a.vx_o / a.vz_o (a step from one state
-// buffer into another); else in place.
-template <typename T, bool PP, bool OOP, bool HINT>
+// buffer into another); else in place.  RAG: nx % 4 != 0, the last group of
+// a row reaches past the update region (an instantiation of its own: keeping
+// the old velocities for it cost the others 0.7 % of a TTI step).
+template <typename T, bool PP, bool OOP, bool HINT, bool RAG>
 __device__ __forceinline__ void split_vel_finish(const StepArgs<T> &a, const FusedExtras<T> &x, int tile,
                                                  int gi0, int gj, long long g, const Q4<T> &vxi,
                                                  const Q4<T> &vzi, const Q4<T> &r0, const Q4<T> &r1, T r4,
@@ -66,6 +68,10 @@ __device__ __forceinline__ void split_vel_finish(const StepArgs<T> &a, const Fus
     else
       add_lane4(vzn, k, a.dt * two_over_s(lane4(r0, k) + lane4(r1, k)) * f);
   }
+  if (RAG && gi0 + 4 > nx - L) {
+    keep_edge4(vxn, nx - L - gi0, vxi.v);
+    keep_edge4(vzn, nx - L - gi0, vzi.v);
+  }
   // v is re-read by the stress pass of the same step: keep it in L2
   sth4((OOP ? a.vx_o : a.vx) + g, vxn, l2_keep_c<HINT>());
   sth4((OOP ? a.vz_o : a.vz) + g, vzn, l2_keep_c<HINT>());
@@ -85,7 +91,7 @@ __device__ __forceinline__ void split_vel_sample(const StepArgs<T> &a, const Fus
   for (int e = e0 + (int)threadIdx.x; e < e1; e += (int)blockDim.x) {
     const int4 en = x.tile_ent[e];
     if (en.w != TL_RECEIVER) continue;
-    const long long c = (long long)en.y * a.nx + en.x;
+    const long long c = (long long)en.y * a.ld + en.x;
     x.traces[(long long)en.z * x.tnt + x.it] = vx[c];
     x.traces[(long long)(x.nrec + en.z) * x.tnt + x.it] = vz[c];
   }
@@ -95,22 +101,22 @@ __device__ __forceinline__ void split_vel_sample(const StepArgs<T> &a, const Fus
 // else in place on the input set.  OOP (implies PP): v written to the
 // output state too.  AFDA: the grid has the H-AFDA free surface (a
 // separate instantiation, so the others carry none of its registers).
-template <typename T, bool PP, bool OOP, bool HINT, bool AFDA = false>
+template <typename T, bool PP, bool OOP, bool HINT, bool AFDA = false, bool RAG = false>
 __device__ __forceinline__ void split_vel_tile(const StepArgs<T> &a, const FusedExtras<T> &x,
                                                int tile) {
   using G = SplitGeom<T>;
   constexpr int TX = G::TX, TZ = G::TZ;
   T *const psix_o = PP ? a.psix_o : a.psix, *const psiz_o = PP ? a.psiz_o : a.psiz;
   const int x0 = L + (tile % x.ntx) * TX, z0 = L + (tile / x.ntx) * TZ;
-  const int nx = a.nx, nz = a.nz, xe = nx - L, ze = nz - L;
+  const int ld = a.ld, xe = a.nx - L, ze = a.nz - L;
   const int tid = threadIdx.x;
   const int r = tid / (TX / 4), lx = 4 * (tid % (TX / 4));
   const int gi0 = x0 + lx, gj = z0 + r;
   if (gi0 >= xe || gj >= ze) return;
-  const long long g = (long long)gj * nx + gi0;
+  const long long g = (long long)gj * ld + gi0;
   const Q4<T> vxi = ldc4(a.vx + g), vzi = ldc4(a.vz + g);
   const int e0 = x.tile_off[tile], e1 = x.tile_off[tile + 1];
-  const Q4<T> r0 = ldg4(a.rho + g), r1 = ldg4(a.rho + g + nx);
+  const Q4<T> r0 = ldg4(a.rho + g), r1 = ldg4(a.rho + g + ld);
   const T r4 = __ldg(a.rho + g + 4);
   T hxx[12], hxz[12];
 #pragma unroll
@@ -127,21 +133,21 @@ __device__ __forceinline__ void split_vel_tile(const StepArgs<T> &a, const Fused
   for (int q = -4; q <= 4; ++q) {
     if (q <= 3) {  // ddzm(sxz)
       const T cq = q >= 0 ? a.Dz[q] : -a.Dz[-q - 1];
-      const Q4<T> v = q == 0 ? win4(hxz, 4) : ldg4(a.sxz + g + (long long)q * nx);
+      const Q4<T> v = q == 0 ? win4(hxz, 4) : ldg4(a.sxz + g + (long long)q * ld);
       zxz = fma4(splat4<T>(cq), v, zxz);
     }
     if (q >= -3) {  // ddzp(szz)
       const T cq = q >= 1 ? a.Dz[q - 1] : -a.Dz[-q];
-      const Q4<T> v = ldg4(a.szz + g + (long long)q * nx);
+      const Q4<T> v = ldg4(a.szz + g + (long long)q * ld);
       zzz = fma4(splat4<T>(cq), v, zzz);
     }
   }
   if (AFDA && gj < L + 4) {  // one-sided z derivatives below the H-AFDA surface
     const int qs = gj - L;
-    zxz = afda4<0>(a, qs, [&](int m) { return ldg4(a.sxz + (long long)(L + m) * nx + gi0); });
-    if (qs < 3) zzz = afda4<1>(a, qs, [&](int m) { return ldg4(a.szz + (long long)(L + 1 + m) * nx + gi0); });
+    zxz = afda4<0>(a, qs, [&](int m) { return ldg4(a.sxz + (long long)(L + m) * ld + gi0); });
+    if (qs < 3) zzz = afda4<1>(a, qs, [&](int m) { return ldg4(a.szz + (long long)(L + 1 + m) * ld + gi0); });
   }
-  split_vel_finish<T, PP, OOP, HINT>(a, x, tile, gi0, gj, g, vxi, vzi, r0, r1, r4, hxx, hxz, zxz, zzz, psix_o, psiz_o,
+  split_vel_finish<T, PP, OOP, HINT, RAG>(a, x, tile, gi0, gj, g, vxi, vzi, r0, r1, r4, hxx, hxz, zxz, zzz, psix_o, psiz_o,
                                      e0, e1);
 }
 
@@ -172,7 +178,7 @@ struct SplitVelTmaT {
 template <typename T>
 using SplitVelTma = SplitVelTmaT<T>;
 
-template <typename T, bool PP, bool HINT, bool AFDA, typename G = SplitVelTma<T>>
+template <typename T, bool PP, bool HINT, bool AFDA, bool RAG = false, typename G = SplitVelTma<T>>
 __device__ __forceinline__ void split_vel_tma_tile(const StepArgs<T> &a, const FusedExtras<T> &x,
                                                    const SplitMaps &maps, int tile) {
   constexpr int TX = G::TX, WX = G::WX, WZ = G::WZ;
@@ -183,7 +189,7 @@ __device__ __forceinline__ void split_vel_tma_tile(const StepArgs<T> &a, const F
   const T *s_szz = reinterpret_cast<T *>(smem_raw) + G::O_SZZ;
   T *const psix_o = PP ? a.psix_o : a.psix, *const psiz_o = PP ? a.psiz_o : a.psiz;
   const int x0 = L + (tile % x.ntx) * TX, z0 = L + (tile / x.ntx) * G::TZ;
-  const int nx = a.nx, nz = a.nz, xe = nx - L, ze = nz - L;
+  const int ld = a.ld, xe = a.nx - L, ze = a.nz - L;
   const int tid = threadIdx.x;
   if (tid == 0) mbar_init(bar, 1);
   __syncthreads();
@@ -197,7 +203,7 @@ __device__ __forceinline__ void split_vel_tma_tile(const StepArgs<T> &a, const F
   const int r = tid / (TX / 4), lx = 4 * (tid % (TX / 4));
   const int gi0 = x0 + lx, gj = z0 + r;
   const bool act = gi0 < xe && gj < ze;
-  const long long g = (long long)gj * nx + gi0;
+  const long long g = (long long)gj * ld + gi0;
   // the other threads read v (last written by the previous velocity pass,
   // complete before the stress pass that precedes this grid was released)
   // and rho while that stress pass may still drain; sigma comes by TMA
@@ -208,7 +214,7 @@ __device__ __forceinline__ void split_vel_tma_tile(const StepArgs<T> &a, const F
     vxi = ldcg4(a.vx + g);
     vzi = ldcg4(a.vz + g);
     r0 = ldg4(a.rho + g);
-    r1 = ldg4(a.rho + g + nx);
+    r1 = ldg4(a.rho + g + ld);
     r4 = __ldg(a.rho + g + 4);
   }
   const int e0 = x.tile_off[tile], e1 = x.tile_off[tile + 1];  // the tile's sources, while the boxes land
@@ -245,7 +251,7 @@ __device__ __forceinline__ void split_vel_tma_tile(const StepArgs<T> &a, const F
     zxz = afda4<0>(a, qs, [&](int m) { return lds4(s_sxz + (m + 4) * WX + lx + 4); });
     if (qs < 3) zzz = afda4<1>(a, qs, [&](int m) { return lds4(s_szz + (m + 5) * WZ + lx); });
   }
-  split_vel_finish<T, PP, false, HINT>(a, x, tile, gi0, gj, g, vxi, vzi, r0, r1, r4, hxx, hxz, zxz, zzz, psix_o,
+  split_vel_finish<T, PP, false, HINT, RAG>(a, x, tile, gi0, gj, g, vxi, vzi, r0, r1, r4, hxx, hxz, zxz, zzz, psix_o,
                                        psiz_o, e0, e1);
 }
 
@@ -269,7 +275,7 @@ __device__ __forceinline__ void split_stress_tile(const StepArgs<T> &a, const Fu
   T *s_vx = reinterpret_cast<T *>(smem_raw) + G::O0;
   T *s_vz = s_vx + PB;
   const int x0 = L + (tile % x.ntx) * TX, z0 = L + (tile / x.ntx) * TZ;
-  const int nx = a.nx, nz = a.nz, xe = nx - L, ze = nz - L;
+  const int nx = a.nx, nz = a.nz, ld = a.ld, xe = nx - L, ze = nz - L;
   const int tid = threadIdx.x;
   if constexpr (!EARLY) pdl_wait();  // the new velocities are complete and visible
   if (tid == 0) mbar_init(bar, 1);
@@ -285,7 +291,7 @@ __device__ __forceinline__ void split_stress_tile(const StepArgs<T> &a, const Fu
   const int r = tid / (TX / 4), lx = 4 * (tid % (TX / 4));
   const int gi0 = x0 + lx, gj = z0 + r;
   const bool act = gi0 < xe && gj < ze;
-  const long long g = (long long)gj * nx + gi0;
+  const long long g = (long long)gj * ld + gi0;
   // every own-cell operand, issued before the arithmetic
   Q4<T> sxx{}, szz{}, sxz{}, c13{}, c55a{}, c55b{}, c11{}, c33{}, tau{};
   T c55a4 = 0, c55b4 = 0;
@@ -296,9 +302,9 @@ __device__ __forceinline__ void split_stress_tile(const StepArgs<T> &a, const Fu
     sxz = EARLY ? ldcg4(a.sxz + g) : ldc4(a.sxz + g);
     c13 = ldgh4(a.c13 + g, l2_stream_c<HINT>());
     c55a = ldg4(a.c55 + g);
-    c55b = ldg4(a.c55 + g + nx);
+    c55b = ldg4(a.c55 + g + ld);
     c55a4 = __ldg(a.c55 + g + 4);
-    c55b4 = __ldg(a.c55 + g + nx + 4);
+    c55b4 = __ldg(a.c55 + g + ld + 4);
     if constexpr (KIND != VI_MEDIUM_ISO) {
       c11 = ldgh4(a.c11 + g, l2_stream_c<HINT>());
       c33 = ldgh4(a.c33 + g, l2_stream_c<HINT>());
@@ -434,6 +440,11 @@ __device__ __forceinline__ void split_stress_tile(const StepArgs<T> &a, const Fu
     sth_u2(a.slo + 2 * a.slo_plane + g, lxz, l2_stream_c<HINT>());
   }
   if (surf) szz = Q4<T>{{0, 0, 0, 0}};
+  if (gi0 + 4 > xe) {  // ragged last group of a row (its memory variables outside are never read)
+    keep_edge4(sxx, xe - gi0, a.sxx + g);
+    keep_edge4(szz, xe - gi0, a.szz + g);
+    keep_edge4(sxz, xe - gi0, a.sxz + g);
+  }
   if (!finite3(sxx, szz, sxz)) atomicOr(x.err, kErrNonFinite);
   T *const osxx = OOP ? a.sxx_o : a.sxx, *const oszz = OOP ? a.szz_o : a.szz, *const osxz = OOP ? a.sxz_o : a.sxz;
   // sigma is re-read by the next velocity pass: keep it in L2
@@ -447,13 +458,13 @@ __device__ __forceinline__ void split_stress_tile(const StepArgs<T> &a, const Fu
       Q4<T> im;
 #pragma unroll
       for (int q = 0; q < 4; ++q) im.v[q] = -szz.v[q];
-      stg4(oszz + (long long)(L - k) * nx + gi0, im);
+      stg4(oszz + (long long)(L - k) * ld + gi0, im);
     }
     if (k >= 0 && k < L) {
       Q4<T> im;
 #pragma unroll
       for (int q = 0; q < 4; ++q) im.v[q] = -sxz.v[q];
-      stg4(osxz + (long long)(L - 1 - k) * nx + gi0, im);
+      stg4(osxz + (long long)(L - 1 - k) * ld + gi0, im);
     }
   }
 }

@@ -125,7 +125,11 @@ __device__ __forceinline__ Q4<T> mean4_fwd(const Q4<T> &a, T a4, const Q4<T> &b,
 }
 
 // COMP (FP32): sigma accumulated with its rounding residue (a.slo, two_sum_acc4).
-template <typename T, int NSLS, bool HINT, bool COMP = false, bool AFDA = false, typename G = SplitTtiGeom<T>>
+// RAG: nx % 4 != 0, so the last group of a row reaches past the update region
+// (an instantiation of its own: the selects in the others cost 1.3 % of a
+// 1024 x 512 step).
+template <typename T, int NSLS, bool HINT, bool COMP = false, bool AFDA = false, bool RAG = false,
+          typename G = SplitTtiGeom<T>>
 __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, const FusedExtras<T> &x,
                                                       const SplitMaps &maps, int tile) {
   static_assert(!COMP || sizeof(T) == 4, "compensated stress: FP32");
@@ -136,7 +140,7 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
   T *s_vz = s_vx + G::PB;
   T *s_exx = s_vz + G::PB, *s_ezz = s_exx + G::PE, *s_exz = s_ezz + G::PE;
   const int x0 = L + (tile % x.ntx) * TX, z0 = L + (tile / x.ntx) * TZ;
-  const int nx = a.nx, nz = a.nz, xe = nx - L, ze = nz - L;
+  const int ld = a.ld, xe = a.nx - L, ze = a.nz - L;
   const int tid = threadIdx.x;
   pdl_wait();  // the new velocities are complete and visible
   if (tid == 0) mbar_init(bar, 1);
@@ -151,7 +155,7 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
   const int r = tid / (TX / 4), lx = 4 * (tid % (TX / 4));
   const int gi0 = x0 + lx, gj = z0 + r;
   const bool act = gi0 < xe && gj < ze;
-  const long long g = (long long)gj * nx + gi0;
+  const long long g = (long long)gj * ld + gi0;
   Q4<T> tau = splat4<T>(0);
   if (act && NSLS > 0) tau = ldg4(a.tau + g);
   // the ring group of this thread (threads 0 .. NRING-1): e-box row/column
@@ -166,7 +170,7 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
   }
   const int rgi0 = x0 - 4 + rc, rgj = z0 - 1 + rr;
   const bool ract = rr >= 0 && rgi0 >= L && rgi0 < xe && rgj >= L && rgj < ze;
-  const long long rg = (long long)rgj * nx + rgi0;
+  const long long rg = (long long)rgj * ld + rgi0;
   Q4<T> rtau = splat4<T>(0);
   if (ract && NSLS > 0) rtau = ldg4(a.tau + rg);
   // while the box is in flight: the memory-variable sums into registers
@@ -189,6 +193,11 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
     if (act) {
       tti_rates4<T, BW, AFDA>(a, s_vx, s_vz, (r + 5) * BW + lx + 4, gi0, gj, true, rxx, rzz, rxz);
       tti_effective4<T, NSLS>(tau, mxx, mzz, mxz, rxx, rzz, rxz, exx, ezz, exz);
+      if (RAG && gi0 + 4 > xe) {  // zero outside U
+        zero_edge4(exx, xe - gi0);
+        zero_edge4(ezz, xe - gi0);
+        zero_edge4(exz, xe - gi0);
+      }
     }
     const int e = (r + 1) * EW + lx + 4;
     stg4(s_exx + e, exx);
@@ -201,6 +210,11 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
       Q4<T> qxx, qzz, qxz;
       tti_rates4<T, BW, AFDA>(a, s_vx, s_vz, (rr + 4) * BW + rc, rgi0, rgj, false, qxx, qzz, qxz);
       tti_effective4<T, NSLS>(rtau, qmxx, qmzz, qmxz, qxx, qzz, qxz, exx, ezz, exz);
+      if (RAG && rgi0 + 4 > xe) {
+        zero_edge4(exx, xe - rgi0);
+        zero_edge4(ezz, xe - rgi0);
+        zero_edge4(exz, xe - rgi0);
+      }
     }
     const int e = rr * EW + rc;
     stg4(s_exx + e, exx);
@@ -215,7 +229,7 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
       const int gi = x0 + c;
       if (gi >= xe) continue;
       const int e = EW + c + 4;
-      const long long gs = (long long)L * nx + gi;
+      const long long gs = (long long)L * ld + gi;
       const T eb = T(0.25) * (s_exz[e] + s_exz[e - 1] + s_exz[e - EW] + s_exz[e - EW - 1]);
       s_ezz[e] = -(__ldg(a.c13 + gs) * s_exx[e] + __ldg(a.c35 + gs) * eb) / __ldg(a.c33 + gs);
     }
@@ -230,12 +244,12 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
   // read once per step: streamed through L2 (ring-shared operands are not)
   const Q4<T> C11 = ldgh4(a.c11 + g, l2_stream_c<HINT>()), C13 = ldgh4(a.c13 + g, l2_stream_c<HINT>()),
               C33 = ldgh4(a.c33 + g, l2_stream_c<HINT>());
-  const Q4<T> c15a = ldg4(a.c15 + g), c15b = ldg4(a.c15 + g + nx);
-  const Q4<T> c35a = ldg4(a.c35 + g), c35b = ldg4(a.c35 + g + nx);
-  const Q4<T> c55a = ldg4(a.c55 + g), c55b = ldg4(a.c55 + g + nx);
-  const T c15a4 = __ldg(a.c15 + g + 4), c15b4 = __ldg(a.c15 + g + nx + 4);
-  const T c35a4 = __ldg(a.c35 + g + 4), c35b4 = __ldg(a.c35 + g + nx + 4);
-  const T c55a4 = __ldg(a.c55 + g + 4), c55b4 = __ldg(a.c55 + g + nx + 4);
+  const Q4<T> c15a = ldg4(a.c15 + g), c15b = ldg4(a.c15 + g + ld);
+  const Q4<T> c35a = ldg4(a.c35 + g), c35b = ldg4(a.c35 + g + ld);
+  const Q4<T> c55a = ldg4(a.c55 + g), c55b = ldg4(a.c55 + g + ld);
+  const T c15a4 = __ldg(a.c15 + g + 4), c15b4 = __ldg(a.c15 + g + ld + 4);
+  const T c35a4 = __ldg(a.c35 + g + 4), c35b4 = __ldg(a.c35 + g + ld + 4);
+  const T c55a4 = __ldg(a.c55 + g + 4), c55b4 = __ldg(a.c55 + g + ld + 4);
   const int e = (r + 1) * EW + lx + 4;
   const Q4<T> exx = lds4(s_exx + e), ezz = lds4(s_ezz + e), exz = lds4(s_exz + e);
   // e_xz at the integer node: mean of (i-1/2, j-1/2) .. (i+1/2, j+1/2)
@@ -295,6 +309,11 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
     sth_u2(a.slo + 2 * a.slo_plane + g, lxz, l2_stream_c<HINT>());
   }
   if (surf) szz = splat4<T>(0);
+  if (RAG && gi0 + 4 > xe) {  // (its memory variables outside are never read)
+    keep_edge4(sxx, xe - gi0, a.sxx + g);
+    keep_edge4(szz, xe - gi0, a.szz + g);
+    keep_edge4(sxz, xe - gi0, a.sxz + g);
+  }
   if (!finite3(sxx, szz, sxz)) atomicOr(x.err, kErrNonFinite);
   // sigma is re-read by the next velocity pass: keep it in L2
   sth4(a.sxx + g, sxx, l2_keep_c<HINT>());
@@ -303,16 +322,16 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
   if (x.fs == kFsImaging) {
     // stress images: szz(L-k) = -szz(L+k), k = 1..4; sxz(L-1-k) = -sxz(L+k), k = 0..3
     const int k = gj - L;
-    if (k >= 1 && k <= L) stg4(a.szz + (long long)(L - k) * nx + gi0, mul4(splat4<T>(T(-1)), szz));
-    if (k >= 0 && k < L) stg4(a.sxz + (long long)(L - 1 - k) * nx + gi0, mul4(splat4<T>(T(-1)), sxz));
+    if (k >= 1 && k <= L) stg4(a.szz + (long long)(L - k) * ld + gi0, mul4(splat4<T>(T(-1)), szz));
+    if (k >= 0 && k < L) stg4(a.sxz + (long long)(L - 1 - k) * ld + gi0, mul4(splat4<T>(T(-1)), sxz));
   }
 }
 
-template <typename T, int NSLS, bool HINT, bool COMP, bool AFDA>
+template <typename T, int NSLS, bool HINT, bool COMP, bool AFDA, bool RAG>
 __global__ void __launch_bounds__(SplitTtiGeom<T>::NT, (sizeof(T) == 4 ? 512 : 256) / SplitTtiGeom<T>::NT)
     k_split_stress_tti(const __grid_constant__ StepArgs<T> a, const __grid_constant__ FusedExtras<T> x,
                        const __grid_constant__ SplitMaps maps) {
-  split_stress_tti_tile<T, NSLS, HINT, COMP, AFDA>(a, x, maps, blockIdx.x);
+  split_stress_tti_tile<T, NSLS, HINT, COMP, AFDA, RAG>(a, x, maps, blockIdx.x);
 }
 
 // Batched: one tile of one shot per CTA; the step parity selects the
@@ -328,12 +347,12 @@ __global__ void __launch_bounds__(SplitTtiGeomBatch<T>::NT, (sizeof(T) == 4 ? 51
   // split step; AFDA: some shot has the H-AFDA surface
   using G = SplitTtiGeomBatch<T>;
   if (AFDA && x.fs == kFsAfda)
-    split_stress_tti_tile<T, NSLS, false, COMP, true, G>(b.args[2 * shot + (it & 1)], x, b.smaps[shot], tile);
+    split_stress_tti_tile<T, NSLS, false, COMP, true, false, G>(b.args[2 * shot + (it & 1)], x, b.smaps[shot], tile);
   else
-    split_stress_tti_tile<T, NSLS, false, COMP, false, G>(b.args[2 * shot + (it & 1)], x, b.smaps[shot], tile);
+    split_stress_tti_tile<T, NSLS, false, COMP, false, false, G>(b.args[2 * shot + (it & 1)], x, b.smaps[shot], tile);
 }
 
-template <typename T, int NSLS, bool HINT, bool COMP = false, bool AFDA = false>
+template <typename T, int NSLS, bool HINT, bool COMP = false, bool AFDA = false, bool RAG = false>
 static int launch_tti_k(const StepArgs<T> &a, const FusedExtras<T> &x, const SplitMaps &m, int ntiles,
                         cudaStream_t st, bool pdl) {
   using G = SplitTtiGeom<T>;
@@ -341,12 +360,12 @@ static int launch_tti_k(const StepArgs<T> &a, const FusedExtras<T> &x, const Spl
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(attr_set & (1ULL << dev))) {
-    cudaError_t e = cudaFuncSetAttribute(k_split_stress_tti<T, NSLS, HINT, COMP, AFDA>,
+    cudaError_t e = cudaFuncSetAttribute(k_split_stress_tti<T, NSLS, HINT, COMP, AFDA, RAG>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
     if (e != cudaSuccess) return cuda_check(e, "split TTI stress smem attribute");
     attr_set |= 1ULL << dev;
   }
-  return cuda_check(launch_pdl(k_split_stress_tti<T, NSLS, HINT, COMP, AFDA>, dim3(ntiles), dim3(G::NT),
+  return cuda_check(launch_pdl(k_split_stress_tti<T, NSLS, HINT, COMP, AFDA, RAG>, dim3(ntiles), dim3(G::NT),
                                (size_t)G::SMEM, st, pdl, a, x, m),
                     "split TTI stress launch");
 }
@@ -355,6 +374,9 @@ static int launch_tti_k(const StepArgs<T> &a, const FusedExtras<T> &x, const Spl
 template <typename T, int NSLS>
 static int launch_tti(const StepArgs<T> &a, const FusedExtras<T> &x, const SplitMaps &m, int ntiles,
                       cudaStream_t st, bool pdl) {
+  if (a.nx % 4 != 0)  // padded planes: plain FP32 or FP64, imaging surface or none
+    return x.l2hint ? launch_tti_k<T, NSLS, true, false, false, true>(a, x, m, ntiles, st, pdl)
+                    : launch_tti_k<T, NSLS, false, false, false, true>(a, x, m, ntiles, st, pdl);
   if constexpr (sizeof(T) == 4) {
     if (a.slo) {
       if (x.fs == kFsAfda)

@@ -313,6 +313,20 @@ __device__ __forceinline__ bool finite3(const Q4<T> &a, const Q4<T> &b, const Q4
   const Q4<T> s = add4(add4(a, b), c);
   return isfinite((s.v[0] + s.v[1]) + (s.v[2] + s.v[3]));
 }
+// the first n lanes of q, the rest from p[0..3]: a 4-cell group that reaches
+// past the update region keeps what its outer cells hold
+template <typename T>
+__device__ __forceinline__ void keep_edge4(Q4<T> &q, int n, const T *p) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (k >= n) q.v[k] = p[k];
+}
+template <typename T>
+__device__ __forceinline__ void zero_edge4(Q4<T> &q, int n) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (k >= n) q.v[k] = T(0);
+}
 // window of 4 consecutive values of a 12-value row, starting at o
 template <typename T>
 __device__ __forceinline__ Q4<T> win4(const T (&u)[12], int o) {

@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kWaveThreads, (sizeof(T) == 4 ? 512 : 256) / k
       FusedExtras<T> x = xv;
       x.it = s;
       const int tile = b * w.ntx_v + u;
-      split_vel_tma_tile<T, false, false, false, WaveVelGeom<T>>(a, x, mv, tile);
+      split_vel_tma_tile<T, false, false, false, false, WaveVelGeom<T>>(a, x, mv, tile);
       split_vel_sample<T>(a, x, tile);
     } else {
       FusedExtras<T> x = xs;
