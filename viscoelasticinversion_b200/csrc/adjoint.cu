@@ -15,6 +15,10 @@
 // psi' = b psi + a d, d~ = d/kappa + psi' transposes to
 // dbar = dbar~/kappa + a (psibar' + dbar~), psibar = b (psibar' + dbar~).
 //
+// The reverse sweep runs on 16-byte groups of cells from TMA boxes; every plane
+// of the workspace has rows of a multiple of 4 cells, whatever the grid's, and
+// the forward sweeps step the split pair on the same slots.
+//
 // Memory: the state (v, sigma, M and the current psi set) is stored every
 // K (default ceil(sqrt(nt))) steps; each segment is recomputed forward into
 // K + 1 state slots and walked backwards.  Wavefields and the adjoint state
@@ -26,15 +30,16 @@
 // dJ/dmu.  vi_gradient_velocity maps them to (vp, vs, rho, 1/Q) and, for
 // VTI, vi_gradient_thomsen to the Thomsen (epsilon, delta).
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "fused.cuh"
 #include "nvtx.cuh"
 #include "fused_tma.cuh"
 #include "pdl.cuh"
-#include "plain.cuh"
 #include "plan.cuh"
 #include "split.cuh"
+#include "tma.cuh"
 #include "vec.cuh"
 
 namespace vb {
@@ -43,8 +48,8 @@ namespace {
 
 template <typename T>
 struct AdjArgs {
-  int nx, nz, nsls, kind, fs;
-  int Lx, Rx, Tz, Bz, wx, hz;
+  int nx, ld, fs;  // ld: row stride of every plane (nx rounded up to a multiple of 4)
+  int Lx, Rx, Tz, Bz, wx;
   T dt;
   T Dx[4], Dz[4];
   T a1[VI_MAX_SLS], a2[VI_MAX_SLS];
@@ -52,6 +57,8 @@ struct AdjArgs {
   const T *c15, *c35;  // TTI couplings
   const T *tx, *tz;
   long long np, psix_plane, psiz_plane;
+  int nz;
+  int keep_bar;  // rbar and dbar fit in half the L2: kept there between their kernels
 };
 
 // one state slot: [vx vz sxx szz sxz M(3N)] planes, then one psi set
@@ -69,239 +76,808 @@ struct Slot {
   __host__ __device__ T *m() const { return base + 5 * np; }
   __host__ __device__ T *psix() const { return base + (5 + 3 * nsls) * np; }
   __host__ __device__ T *psiz() const { return psix() + 4 * px; }
-  // rounded up to 64 elements, so every slot (and, with nx % 4 == 0, every
-  // plane of it) starts on a 16-byte boundary, as the split kernels need
+  // rounded up to 64 elements, so every slot (and every plane of it, rows
+  // being a multiple of 4 cells) starts on a 16-byte boundary
   __host__ __device__ static long long size(long long np, long long px, long long pz, int nsls) {
     return ((5 + 3 * nsls) * np + 4 * px + 4 * pz + 63) / 64 * 64;
   }
 };
 
+// FP64 accumulator planes of the adjoint sweep, each cell its own terms; the
+// planes of half-node or buoyancy terms (H, Q) are spread over the cells they
+// average once, at the end (k_adj_finish).  H and TAU carry the factor dt, the
+// others get it there.
+enum { ACC_HX = 0, ACC_HZ = 1, ACC_TAU = 2, ACC_Q55 = 3, ACC_11 = 4, ACC_13 = 5, ACC_33 = 6,
+       ACC_15 = 7, ACC_35 = 8, ACC_Q15 = 9, ACC_Q35 = 10 };
+// ISO: C11 = C33 = lambda + 2 mu share plane ACC_11
+inline int acc_planes(int kind) { return kind == VI_MEDIUM_TTI ? 11 : kind == VI_MEDIUM_VTI ? 7 : 6; }
+
+// ---- V cells (16 bytes) of a row: 4 FP32 or 2 FP64 ------------------------
 template <typename T>
-__device__ __forceinline__ T tap_p(const T *u, long long c, long long s, const T *D) {  // ddxp/ddzp
-  T v = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) v += D[k] * (u[c + (k + 1) * s] - u[c - k * s]);
-  return v;
+struct VecW {
+  static constexpr int V = 16 / (int)sizeof(T);
+};
+template <typename T>
+struct Pk {
+  T v[VecW<T>::V];
+};
+__device__ __forceinline__ Pk<float> ldv(const float *p) {
+  const float4 q = *reinterpret_cast<const float4 *>(p);
+  return {{q.x, q.y, q.z, q.w}};
+}
+__device__ __forceinline__ Pk<double> ldv(const double *p) {
+  const double2 q = *reinterpret_cast<const double2 *>(p);
+  return {{q.x, q.y}};
+}
+// Operands the kernel only reads: the non-coherent path, so their loads are
+// not ordered behind its stores; volatile, so none moves ahead of pdl_wait().
+__device__ __forceinline__ Pk<float> ldn(const float *p) {
+  Pk<float> q;
+  asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(q.v[0]), "=f"(q.v[1]), "=f"(q.v[2]), "=f"(q.v[3])
+               : "l"(p));
+  return q;
+}
+__device__ __forceinline__ Pk<double> ldn(const double *p) {
+  Pk<double> q;
+  asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(q.v[0]), "=d"(q.v[1]) : "l"(p));
+  return q;
+}
+// state of the kernel before last, ahead of the PDL wait: read at L2
+__device__ __forceinline__ Pk<float> ldcgv(const float *p) {
+  const float4 q = __ldcg(reinterpret_cast<const float4 *>(p));
+  return {{q.x, q.y, q.z, q.w}};
+}
+__device__ __forceinline__ Pk<double> ldcgv(const double *p) {
+  const double2 q = __ldcg(reinterpret_cast<const double2 *>(p));
+  return {{q.x, q.y}};
+}
+__device__ __forceinline__ float ldn1(const float *p) {
+  float q;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(q) : "l"(p));
+  return q;
+}
+__device__ __forceinline__ double ldn1(const double *p) {
+  double q;
+  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(q) : "l"(p));
+  return q;
+}
+__device__ __forceinline__ void stv(float *p, const Pk<float> &q) {
+  *reinterpret_cast<float4 *>(p) = make_float4(q.v[0], q.v[1], q.v[2], q.v[3]);
+}
+__device__ __forceinline__ void stv(double *p, const Pk<double> &q) {
+  *reinterpret_cast<double2 *>(p) = make_double2(q.v[0], q.v[1]);
+}
+// the same with an L2 eviction policy
+__device__ __forceinline__ Pk<float> ldnp(const float *p, uint64_t pol) {
+  Pk<float> q;
+  asm volatile("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=f"(q.v[0]), "=f"(q.v[1]), "=f"(q.v[2]), "=f"(q.v[3])
+               : "l"(p), "l"(pol));
+  return q;
+}
+__device__ __forceinline__ Pk<double> ldnp(const double *p, uint64_t pol) {
+  Pk<double> q;
+  asm volatile("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
+               : "=d"(q.v[0]), "=d"(q.v[1])
+               : "l"(p), "l"(pol));
+  return q;
+}
+__device__ __forceinline__ void stvp(float *p, const Pk<float> &q, uint64_t pol) {
+  asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p), "f"(q.v[0]), "f"(q.v[1]),
+               "f"(q.v[2]), "f"(q.v[3]), "l"(pol)
+               : "memory");
+}
+__device__ __forceinline__ void stvp(double *p, const Pk<double> &q, uint64_t pol) {
+  asm volatile("st.global.L2::cache_hint.v2.f64 [%0], {%1, %2}, %3;" ::"l"(p), "d"(q.v[0]), "d"(q.v[1]), "l"(pol)
+               : "memory");
 }
 template <typename T>
-__device__ __forceinline__ T tap_m(const T *u, long long c, long long s, const T *D) {  // ddxm/ddzm
-  T v = 0;
+__device__ __forceinline__ Pk<T> splat(T s) {
+  Pk<T> r;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) v += D[k] * (u[c + k * s] - u[c - (k + 1) * s]);
-  return v;
+  for (int k = 0; k < VecW<T>::V; ++k) r.v[k] = s;
+  return r;
 }
-// bounds-checked forms for the transposes (u is zero outside its region)
+__device__ __forceinline__ Pk<float> pfma(const Pk<float> &a, const Pk<float> &b, const Pk<float> &c) {
+  const float2 l = __ffma2_rn(make_float2(a.v[0], a.v[1]), make_float2(b.v[0], b.v[1]), make_float2(c.v[0], c.v[1]));
+  const float2 h = __ffma2_rn(make_float2(a.v[2], a.v[3]), make_float2(b.v[2], b.v[3]), make_float2(c.v[2], c.v[3]));
+  return {{l.x, l.y, h.x, h.y}};
+}
+__device__ __forceinline__ Pk<double> pfma(const Pk<double> &a, const Pk<double> &b, const Pk<double> &c) {
+  return {{fma(a.v[0], b.v[0], c.v[0]), fma(a.v[1], b.v[1], c.v[1])}};
+}
+__device__ __forceinline__ Pk<float> pmul(const Pk<float> &a, const Pk<float> &b) {
+  const float2 l = __fmul2_rn(make_float2(a.v[0], a.v[1]), make_float2(b.v[0], b.v[1]));
+  const float2 h = __fmul2_rn(make_float2(a.v[2], a.v[3]), make_float2(b.v[2], b.v[3]));
+  return {{l.x, l.y, h.x, h.y}};
+}
+__device__ __forceinline__ Pk<double> pmul(const Pk<double> &a, const Pk<double> &b) {
+  return {{a.v[0] * b.v[0], a.v[1] * b.v[1]}};
+}
+__device__ __forceinline__ Pk<float> padd(const Pk<float> &a, const Pk<float> &b) {
+  const float2 l = __fadd2_rn(make_float2(a.v[0], a.v[1]), make_float2(b.v[0], b.v[1]));
+  const float2 h = __fadd2_rn(make_float2(a.v[2], a.v[3]), make_float2(b.v[2], b.v[3]));
+  return {{l.x, l.y, h.x, h.y}};
+}
+__device__ __forceinline__ Pk<double> padd(const Pk<double> &a, const Pk<double> &b) {
+  return {{a.v[0] + b.v[0], a.v[1] + b.v[1]}};
+}
 template <typename T>
-__device__ __forceinline__ T tap_p_b(const T *u, int i, int j, int nx, int nz, int ax, const T *D) {
-  T v = 0;
+__device__ __forceinline__ Pk<T> psub(const Pk<T> &a, const Pk<T> &b) {
+  return pfma(b, splat<T>(T(-1)), a);
+}
+template <typename T>
+__device__ __forceinline__ Pk<T> pscale(T s, const Pk<T> &a) {
+  return pmul(splat<T>(s), a);
+}
+// out[k] = term(k, in[k]), FP64: an accumulator plane read from its staged
+// tile and written straight back (32-byte stores for FP32's four cells)
+__device__ __forceinline__ void st_acc(double *p, const double (&t)[4]) {
+  asm volatile("st.global.L2::cache_hint.v4.f64 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p), "d"(t[0]), "d"(t[1]), "d"(t[2]), "d"(t[3]), "l"(l2_stream())
+               : "memory");
+}
+__device__ __forceinline__ void st_acc(double *p, const double (&t)[2]) {
+  *reinterpret_cast<double2 *>(p) = make_double2(t[0], t[1]);
+}
+template <typename T, typename F>
+__device__ __forceinline__ void acc_add(const double *in, double *out, F term) {
+  constexpr int V = VecW<T>::V;
+  double t[V];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int a = k + 1, b = -k;
-    const int ia = ax == 0 ? i + a : i, ja = ax == 0 ? j : j + a;
-    const int ib = ax == 0 ? i + b : i, jb = ax == 0 ? j : j + b;
-    const T ua = (ia >= 0 && ia < nx && ja >= 0 && ja < nz) ? u[(long long)ja * nx + ia] : T(0);
-    const T ub = (ib >= 0 && ib < nx && jb >= 0 && jb < nz) ? u[(long long)jb * nx + ib] : T(0);
-    v += D[k] * (ua - ub);
+  for (int q = 0; q < V; q += 2) {
+    const double2 u = *reinterpret_cast<const double2 *>(in + q);
+    t[q] = term(q, u.x);
+    t[q + 1] = term(q + 1, u.y);
   }
-  return v;
-}
-template <typename T>
-__device__ __forceinline__ T tap_m_b(const T *u, int i, int j, int nx, int nz, int ax, const T *D) {
-  T v = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int a = k, b = -(k + 1);
-    const int ia = ax == 0 ? i + a : i, ja = ax == 0 ? j : j + a;
-    const int ib = ax == 0 ? i + b : i, jb = ax == 0 ? j : j + b;
-    const T ua = (ia >= 0 && ia < nx && ja >= 0 && ja < nz) ? u[(long long)ja * nx + ia] : T(0);
-    const T ub = (ib >= 0 && ib < nx && jb >= 0 && jb < nz) ? u[(long long)jb * nx + ib] : T(0);
-    v += D[k] * (ua - ub);
-  }
-  return v;
+  st_acc(out, t);
 }
 
-// CPML forward at one derivative: returns d~ (and the new psi in *pn)
+// Staggered derivatives of a plane (staged in shared memory, row stride ld)
+// at the group at u.
 template <typename T>
-__device__ __forceinline__ T cpml_fwd(T d, T p0, T a, T b, T ik, T *pn) {
-  const T p = b * p0 + a * d;
-  *pn = p;
-  return d * ik + p;
+struct RowWin {  // u[c - 4 .. c + V + 3]
+  T w[VecW<T>::V + 8];
+};
+template <typename T>
+__device__ __forceinline__ RowWin<T> ldwin(const T *u) {
+  constexpr int V = VecW<T>::V;
+  RowWin<T> r;
+#pragma unroll
+  for (int q = 0; q < (V + 8) / V; ++q) {
+    const Pk<T> t = ldv(u - 4 + V * q);
+#pragma unroll
+    for (int k = 0; k < V; ++k) r.w[V * q + k] = t.v[k];
+  }
+  return r;
+}
+template <typename T>
+__device__ __forceinline__ Pk<T> at(const RowWin<T> &r, int o) {
+  Pk<T> t;
+#pragma unroll
+  for (int k = 0; k < VecW<T>::V; ++k) t.v[k] = r.w[4 + o + k];
+  return t;
+}
+template <typename T>
+__device__ __forceinline__ Pk<T> dxp(const RowWin<T> &r, const T *D) {
+  Pk<T> s = pscale(D[0], psub(at(r, 1), at(r, 0)));
+#pragma unroll
+  for (int q = 1; q < 4; ++q) s = pfma(splat<T>(D[q]), psub(at(r, q + 1), at(r, -q)), s);
+  return s;
+}
+template <typename T>
+__device__ __forceinline__ Pk<T> dxm(const RowWin<T> &r, const T *D) {
+  Pk<T> s = pscale(D[0], psub(at(r, 0), at(r, -1)));
+#pragma unroll
+  for (int q = 1; q < 4; ++q) s = pfma(splat<T>(D[q]), psub(at(r, q), at(r, -q - 1)), s);
+  return s;
+}
+template <typename T>
+__device__ __forceinline__ Pk<T> dzp(const T *u, int ld, const T *D) {
+  Pk<T> s = pscale(D[0], psub(ldv(u + ld), ldv(u)));
+#pragma unroll
+  for (int q = 1; q < 4; ++q) s = pfma(splat<T>(D[q]), psub(ldv(u + (q + 1) * ld), ldv(u - q * ld)), s);
+  return s;
+}
+template <typename T>
+__device__ __forceinline__ Pk<T> dzm(const T *u, int ld, const T *D) {
+  Pk<T> s = pscale(D[0], psub(ldv(u), ldv(u - ld)));
+#pragma unroll
+  for (int q = 1; q < 4; ++q) s = pfma(splat<T>(D[q]), psub(ldv(u + q * ld), ldv(u - (q + 1) * ld)), s);
+  return s;
 }
 
-// ---- images^T: fold the ghost-row adjoints into the rows they mirror ----
-// (all eight rows of a column are loaded before any store: the ghost and
-// target rows are distinct, so the read-modify-writes need not serialise)
+// The CPML strips a group touches.  Profiles outside a strip are 1/kappa =
+// 1, a = b = 0 and psi counts as zero there, so one vector form serves groups
+// that straddle a strip's edge; only groups whose psi cells do not lie on a
+// vector boundary load and store them cell by cell.
 template <typename T>
-__global__ void k_mirror_t(T *sb_zz, T *sb_xz, int nx) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nx) return;
-  T gz[L], tz[L], gq[L], tq[L];
+struct Strips {
+  bool x, z, xvec;
+  int xs[VecW<T>::V];
+  long long xo, zo;
+};
+template <typename T>
+__device__ __forceinline__ Strips<T> strips_of(const AdjArgs<T> &A, int gi0, int j) {
+  constexpr int V = VecW<T>::V;
+  Strips<T> s;
+  s.x = gi0 < A.Lx || gi0 + V - 1 >= A.nx - A.Rx;
+  const int zs = strip_z(j, A.nz, A.Tz, A.Bz);
+  s.z = zs >= 0;
+  s.zo = (long long)zs * A.ld + gi0;
+  s.xo = (long long)j * A.wx;
+  s.xvec = false;
+  if (s.x) {
 #pragma unroll
-  for (int k = 1; k <= L; ++k) {
-    gz[k - 1] = sb_zz[(long long)(L - k) * nx + i];
-    tz[k - 1] = sb_zz[(long long)(L + k) * nx + i];
+    for (int k = 0; k < V; ++k) s.xs[k] = strip_x(gi0 + k, A.nx, A.Lx, A.Rx);
+    s.xvec = s.xs[0] >= 0 && s.xs[V - 1] == s.xs[0] + V - 1 &&
+             (((s.xo + s.xs[0]) | A.psix_plane | A.nx) & (V - 1)) == 0;
+  }
+  return s;
+}
+template <typename T>
+__device__ __forceinline__ Pk<T> ld_psix(const Strips<T> &s, const T *plane) {
+  if (s.xvec) return ldv(plane + s.xo + s.xs[0]);
+  Pk<T> r;
+#pragma unroll
+  for (int k = 0; k < VecW<T>::V; ++k) r.v[k] = s.xs[k] >= 0 ? plane[s.xo + s.xs[k]] : T(0);
+  return r;
+}
+template <typename T>
+__device__ __forceinline__ Pk<T> ld_psix0(const Strips<T> &s, const T *plane) {  // of a forward state
+  if (s.xvec) return ldn(plane + s.xo + s.xs[0]);
+  Pk<T> r;
+#pragma unroll
+  for (int k = 0; k < VecW<T>::V; ++k) r.v[k] = s.xs[k] >= 0 ? ldn1(plane + s.xo + s.xs[k]) : T(0);
+  return r;
+}
+template <typename T>
+__device__ __forceinline__ void st_psix(const Strips<T> &s, T *plane, const Pk<T> &q) {
+  if (s.xvec) {
+    stv(plane + s.xo + s.xs[0], q);
+    return;
   }
 #pragma unroll
-  for (int k = 0; k < L; ++k) {
-    gq[k] = sb_xz[(long long)(L - 1 - k) * nx + i];
-    tq[k] = sb_xz[(long long)(L + k) * nx + i];
-  }
+  for (int k = 0; k < VecW<T>::V; ++k)
+    if (s.xs[k] >= 0) plane[s.xo + s.xs[k]] = q.v[k];
+}
+template <typename T>
+__device__ __forceinline__ Pk<T> ld_tabx(const AdjArgs<T> &A, const Strips<T> &s, int row, int gi0) {
+  const T *p = A.tx + row * A.nx + gi0;
+  if (s.xvec) return ldn(p);
+  Pk<T> r;
 #pragma unroll
-  for (int k = 1; k <= L; ++k) {
-    sb_zz[(long long)(L + k) * nx + i] = tz[k - 1] - gz[k - 1];
-    sb_zz[(long long)(L - k) * nx + i] = T(0);
-  }
+  for (int k = 0; k < VecW<T>::V; ++k) r.v[k] = ldn1(p + k);
+  return r;
+}
+// Asks for the strips' operands of two x and two z derivatives ahead of the
+// PDL wait (psi of the forward state and of the adjoint, the profiles): a tile
+// in a strip otherwise starts four more rounds of loads after its boxes.
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+template <typename T>
+__device__ __forceinline__ void prefetch_strips(const AdjArgs<T> &A, const Strips<T> &s, int gi0, int j,
+                                                const Slot<T> &x0, const T *pxb, const T *pzb, int px0, int px1,
+                                                int pz0, int pz1) {
+  if (s.x) {
+    const int xs = s.xs[0] >= 0 ? s.xs[0] : s.xs[VecW<T>::V - 1];
+    const long long o0 = px0 * A.psix_plane + s.xo + xs, o1 = px1 * A.psix_plane + s.xo + xs;
+    prefetch_l1(x0.psix() + o0);
+    prefetch_l1(x0.psix() + o1);
+    prefetch_l1(pxb + o0);
+    prefetch_l1(pxb + o1);
 #pragma unroll
-  for (int k = 0; k < L; ++k) {
-    sb_xz[(long long)(L + k) * nx + i] = tq[k] - gq[k];
-    sb_xz[(long long)(L - 1 - k) * nx + i] = T(0);
+    for (int q = 0; q < 6; ++q) prefetch_l1(A.tx + q * A.nx + gi0);
+  }
+  if (s.z) {
+    const long long o0 = pz0 * A.psiz_plane + s.zo, o1 = pz1 * A.psiz_plane + s.zo;
+    prefetch_l1(x0.psiz() + o0);
+    prefetch_l1(x0.psiz() + o1);
+    prefetch_l1(pzb + o0);
+    prefetch_l1(pzb + o1);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) prefetch_l1(A.tz + q * A.nz + j);
+  }
+}
+// forward derivative d -> d/kappa + (b psi + a d), psi of the step's start
+template <typename T>
+__device__ __forceinline__ void cpml_fwd_x(const AdjArgs<T> &A, const Strips<T> &s, int gi0, const T *psix, int pl,
+                                           int tik, int ta, int tb, Pk<T> &d) {
+  const Pk<T> p = pfma(ld_tabx(A, s, tb, gi0), ld_psix0(s, psix + pl * A.psix_plane),
+                       pmul(ld_tabx(A, s, ta, gi0), d));
+  d = pfma(d, ld_tabx(A, s, tik, gi0), p);
+}
+template <typename T>
+__device__ __forceinline__ void cpml_fwd_z(const AdjArgs<T> &A, const Strips<T> &s, int j, const T *psiz, int pl,
+                                           int tik, int ta, int tb, Pk<T> &d) {
+  const Pk<T> p = pfma(splat<T>(A.tz[tb * A.nz + j]), ldn(psiz + pl * A.psiz_plane + s.zo),
+                       pscale(A.tz[ta * A.nz + j], d));
+  d = pfma(d, splat<T>(A.tz[tik * A.nz + j]), p);
+}
+// the transpose: P = psibar + dbar; psibar = b P, dbar = dbar/kappa + a P
+template <typename T>
+__device__ __forceinline__ void cpml_adj_x(const AdjArgs<T> &A, const Strips<T> &s, int gi0, T *psix, int pl, int tik,
+                                           int ta, int tb, Pk<T> &d) {
+  T *q = psix + pl * A.psix_plane;
+  const Pk<T> P = padd(ld_psix(s, (const T *)q), d);
+  st_psix(s, q, pmul(ld_tabx(A, s, tb, gi0), P));
+  d = pfma(d, ld_tabx(A, s, tik, gi0), pmul(ld_tabx(A, s, ta, gi0), P));
+}
+template <typename T>
+__device__ __forceinline__ void cpml_adj_z(const AdjArgs<T> &A, const Strips<T> &s, int j, T *psiz, int pl, int tik,
+                                           int ta, int tb, Pk<T> &d) {
+  T *q = psiz + pl * A.psiz_plane + s.zo;
+  const Pk<T> P = padd(ldv((const T *)q), d);
+  stv(q, pscale(A.tz[tb * A.nz + j], P));
+  d = pfma(d, splat<T>(A.tz[tik * A.nz + j]), pscale(A.tz[ta * A.nz + j], P));
+}
+
+// L2 eviction priorities: dbar and rbar, written by one kernel and read by the
+// next, are kept; the forward states (read once per kernel), the memory
+// variables' adjoints and the accumulators (whose next visit is a whole step
+// later) go first.  Without them 163 MB per 1024 x 512 VTI step reached DRAM;
+// the reverse step 48.5 -> 41 us with 8-row tiles.
+template <typename T>
+__device__ __forceinline__ uint64_t bar_policy(const AdjArgs<T> &A) {
+  return A.keep_bar ? l2_keep() : l2_normal();
+}
+
+// ---- the reverse step ----------------------------------------------------
+// One reverse step of ISO and VTI media is two kernels, of TTI three:
+//
+//   k_adj_stress     sigma adjoint of the step (divergence and images
+//                    transposed, below), then S^T per cell
+//   k_adj_vel        v += -D^T rbar, receiver residuals, V^T per cell
+//
+//   TTI: k_adj_sigma_tti (sigma adjoint, forward effective rates),
+//        k_adj_stress_tti (S^T, a 3 x 3 neighbourhood), k_adj_vel
+//
+// Every stage that reads only its own cell is in the kernel that produces its
+// operands; what crosses cells goes through the planes rbar (strain-rate
+// adjoints) and dbar (stress-divergence adjoints).  The ghost rows above a
+// free surface are never stored: their adjoint is -D^T dbar on rows that hold
+// nothing else, so the rows they mirror add it directly (adj_sigma).  The
+// half-node averages and the buoyancy means are linear and do not change with
+// time, so their transposes are taken once, after the sweep (k_adj_finish).
+//
+// A thread has up to 70 16-byte operands: loaded straight into registers they
+// come in a dozen dependent rounds of L2 latency (k_adj_stress ran 33 us at
+// 1024 x 512, issue slots 15 % busy, 12 us from start to end of a CTA).  One
+// thread therefore requests the tile's boxes by TMA at the start of the CTA,
+// the planes of the kernel before last ahead of the PDL wait; only the
+// per-cell operands read once into few registers (the memory-variable sums,
+// the medium) stay ordinary loads.
+
+// Adjoint tile: rows of 512 bytes, 4 rows, one group of V cells per thread
+// (1024 x 512 VTI, whole reverse step: 40.3 us; 256 bytes x 8 rows 41.8, x 4
+// rows with 64 threads 41.9).
+template <typename T>
+struct AdjGeom {
+  static constexpr int V = VecW<T>::V, TX = 512 / (int)sizeof(T), TZ = 4, NT = TX / V * TZ;
+  static constexpr int WX = TX + 8;      // box with the x taps
+  static constexpr int HZ = TZ + 7;      // box with the z taps of one operator
+  static constexpr int WC = TX + V;      // box with one group to the right
+  static constexpr int E = (int)sizeof(T);
+};
+constexpr int up128(int b) { return (b + 127) / 128 * 128; }
+
+// TMA maps: dbar / rbar with x taps and with z taps, the forward states (all
+// slots one 4D map: column, row, plane, slot), the adjoint planes, the
+// accumulators, c55.  Kernels take the ones they use, in this order.
+struct AdjMaps {
+  CUtensorMap px, pz, st_a, st_b, st_c, own, mem, acc, cc, c2, c3;
+};
+
+// Shared memory of a kernel: the barrier, then its boxes (128-byte aligned).
+template <typename T, int NACC, int NM>
+struct StressSmem {
+  using G = AdjGeom<T>;
+  static constexpr int D0 = 128, D1 = D0 + up128(G::WX * G::TZ * G::E), D2 = D1 + up128(G::TX * G::HZ * G::E),
+                       D3 = D2 + up128(G::WX * G::TZ * G::E), VX = D3 + up128(G::TX * G::HZ * G::E),
+                       VZ = VX + up128(G::WX * G::HZ * G::E), SB = VZ + up128(G::WX * G::HZ * G::E),
+                       MB = SB + 3 * G::TX * G::TZ * G::E, CC = MB + NM * G::TX * G::TZ * G::E,
+                       ACC = CC + up128(G::WC * (G::TZ + 1) * G::E), SIZE = ACC + NACC * G::TX * G::TZ * 8;
+  static constexpr int TAPS = (2 * G::WX * G::TZ + 2 * G::TX * G::HZ) * G::E;  // dbar boxes
+  static constexpr int VBOX = 2 * G::WX * G::HZ * G::E;
+  static constexpr int BYTES = TAPS + VBOX + (3 + NM) * G::TX * G::TZ * G::E + G::WC * (G::TZ + 1) * G::E +
+                               NACC * G::TX * G::TZ * 8;
+};
+template <typename T>
+struct VelSmem {
+  using G = AdjGeom<T>;
+  static constexpr int R0 = 128, R1 = R0 + up128(G::WX * G::TZ * G::E), R2 = R1 + up128(G::TX * G::HZ * G::E),
+                       R3 = R2 + up128(G::TX * G::HZ * G::E), SXX = R3 + up128(G::WX * G::TZ * G::E),
+                       SXZ = SXX + up128(G::WX * G::TZ * G::E), SZZ = SXZ + up128(G::WX * G::HZ * G::E),
+                       VB = SZZ + up128(G::TX * G::HZ * G::E), ACC = VB + 2 * G::TX * G::TZ * G::E,
+                       SIZE = ACC + 2 * G::TX * G::TZ * 8;
+  static constexpr int BYTES = (3 * G::WX * G::TZ + 3 * G::TX * G::HZ + G::WX * G::HZ + 2 * G::TX * G::TZ) * G::E +
+                               2 * G::TX * G::TZ * 8;
+};
+template <typename T>
+struct TtiSmem {  // k_adj_stress_tti: tile and a one-cell ring (x from the group before)
+  using G = AdjGeom<T>;
+  static constexpr int RH = G::TZ + 2, RING = up128(G::WX * RH * G::E), NACC = 9;
+  // the three planes of a 3D box follow each other without padding
+  static constexpr int RP = G::WX * RH * G::E;
+  static constexpr int FE = 128, SB = FE + up128(3 * RP), C15 = SB + up128(3 * RP), C35 = C15 + RING, CC = C35 + RING,
+                       ACC = CC + up128(G::WC * (G::TZ + 1) * G::E), SIZE = ACC + NACC * G::TX * G::TZ * 8;
+  static constexpr int BYTES = 8 * RP + G::WC * (G::TZ + 1) * G::E + NACC * G::TX * G::TZ * 8;
+};
+
+struct AdjTile {
+  int x0, z0, lx, r, gi0, j;
+  bool act;
+};
+template <typename T>
+__device__ __forceinline__ AdjTile adj_tile(const AdjArgs<T> &A, int ntx) {
+  using G = AdjGeom<T>;
+  AdjTile t;
+  const int tile = blockIdx.x;
+  t.r = threadIdx.x / (G::TX / G::V);
+  t.lx = G::V * (threadIdx.x % (G::TX / G::V));
+  t.x0 = L + (tile % ntx) * G::TX;
+  t.z0 = L + (tile / ntx) * G::TZ;
+  t.gi0 = t.x0 + t.lx;
+  t.j = t.z0 + t.r;
+  t.act = t.gi0 < A.nx - L && t.j < A.nz - L;
+  return t;
+}
+// every thread: the boxes have landed (or the wait gave up: kErrTimeout)
+__device__ __forceinline__ bool boxes_landed(uint64_t *bar, int *err) {
+  const bool ok = mbar_wait_bounded(bar, 0, 1u << 22);
+  if (!__syncthreads_or(!ok)) return true;
+  if (threadIdx.x == 0) {
+    atomicOr(err, kErrTimeout);
+    mbar_wait_bounded(bar, 0, 1u << 22);
+  }
+  return false;
+}
+// lanes of a group past the update region (nx % V != 0)
+template <typename T>
+__device__ __forceinline__ void zero_outside(Pk<T> &q, int n) {
+#pragma unroll
+  for (int k = 0; k < VecW<T>::V; ++k)
+    if (k >= n) q.v[k] = T(0);
+}
+// u[k + 1] of the group, u[V] from `next`
+template <typename T>
+__device__ __forceinline__ T right_of(const Pk<T> &u, int k, T next) {
+  constexpr int V = VecW<T>::V;
+  return k + 1 < V ? u.v[k + 1 < V ? k + 1 : 0] : next;
+}
+
+// sigma adjoint before the stress stage of the step: sigma - D^T dbar of the
+// velocity stage after it, with the images transposed: row L + k also takes
+// what -D^T dbar leaves on the ghost rows L - k (szz) and L - 1 - k (sxz),
+// whose only terms are those dbar rows at or below the surface (within four
+// rows of row L + k, so inside its boxes).  sb, d0 .. d3: the group's place in the boxes.
+template <typename T>
+__device__ __forceinline__ void adj_sigma(const AdjArgs<T> &A, const AdjTile &t, const T *sb, const T *d0, const T *d1,
+                                          const T *d2, const T *d3, Pk<T> &bxx, Pk<T> &bzz, Pk<T> &bxz) {
+  using G = AdjGeom<T>;
+  bxx = psub(ldv(sb), dxm(ldwin(d0), A.Dx));
+  bzz = psub(ldv(sb + G::TX * G::TZ), dzm(d3, G::TX, A.Dz));
+  bxz = psub(ldv(sb + 2 * G::TX * G::TZ), padd(dzp(d1, G::TX, A.Dz), dxp(ldwin(d2), A.Dx)));
+  if (A.fs && t.j < 2 * L) {
+    const int k = t.j - L;
+    for (int q = k; q < 4; ++q) {  // grid row L - k + q: 2 k - q rows up from row L + k
+      const T d = A.Dz[q];
+      bxz = pfma(splat<T>(d), ldv(d1 + (q - 2 * k) * G::TX), bxz);
+      if (k >= 1) bzz = pfma(splat<T>(d), ldv(d3 + (q - 2 * k) * G::TX), bzz);
+    }
+  }
+  if (t.gi0 + G::V > A.nx - L) {
+    zero_outside(bxx, A.nx - L - t.gi0);
+    zero_outside(bzz, A.nx - L - t.gi0);
+    zero_outside(bxz, A.nx - L - t.gi0);
   }
 }
 
-// ---- S^T: SLS stress stage transposed, per cell of the update region ----
-// scratch planes: rbar[0..3] = (xx, zz, zx, xz) strain-rate adjoints, q = dt*sxzbar*exz.
-// N (mechanisms) is a template parameter and every operand is loaded
-// before the arithmetic, so the memory-variable and gradient
-// read-modify-writes do not wait on one another.
-template <typename T, int N>
-__global__ void __launch_bounds__(256) k_stress_t(AdjArgs<T> A, Slot<T> x0, Slot<T> x1, Slot<T> ab,
-                                                   T *rbar, T *q, double *gc11, double *gc13,
-                                                   double *gc33, double *gtau) {
-  pdl_wait();  // launched while the previous kernel drains
-  constexpr int NM = N > 0 ? N : 1;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + L;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + L;
-  if (i >= A.nx - L || j >= A.nz - L) return;
-  const int nx = A.nx;
-  const long long c = (long long)j * nx + i, np = A.np;
-  // ---- loads
-  T mo[3 * NM], mbo[3 * NM];
-#pragma unroll
-  for (int k = 0; k < 3 * N; ++k) {
-    mo[k] = x0.m()[k * np + c];
-    mbo[k] = ab.m()[k * np + c];
+// Forward strain rates of the step from the new velocities (vx, vz: the
+// group's place in the boxes) and the CPML memory before it (x0): xx, zz, xz.
+template <typename T>
+__device__ __forceinline__ void adj_rates(const AdjArgs<T> &A, const Slot<T> &x0, const Strips<T> &s, const AdjTile &t,
+                                          const T *vx, const T *vz, Pk<T> (&rt)[3]) {
+  using G = AdjGeom<T>;
+  rt[0] = dxm(ldwin(vx), A.Dx);
+  rt[1] = dzm(vz, G::WX, A.Dz);
+  Pk<T> r3 = dxp(ldwin(vz), A.Dx), r2 = dzp(vx, G::WX, A.Dz);
+  if (s.x) {
+    cpml_fwd_x(A, s, t.gi0, (const T *)x0.psix(), PX_VX, T_IK, T_A, T_B, rt[0]);
+    cpml_fwd_x(A, s, t.gi0, (const T *)x0.psix(), PX_VZ, T_IKH, T_AH, T_BH, r3);
   }
-  T *sbx = ab.sxx(), *sbz = ab.szz(), *sbq = ab.sxz();
-  const T bxx = sbx[c], bzz = sbz[c], bxz = sbq[c];
-  const double g11o = gc11[c], g13o = gc13[c], g33o = gc33[c];
-  const double gto = N > 0 ? gtau[c] : 0.0;
-  const T tau = N > 0 ? A.tau[c] : T(0);
-  const T c13 = A.c13[c], c55 = A.c55[c];
-  const T c11 = A.kind == VI_MEDIUM_ISO ? T(0) : A.c11[c];
-  const T c33 = A.kind == VI_MEDIUM_ISO ? T(0) : A.c33[c];
-  const T c55r = A.c55[c + 1], c55b = A.c55[c + nx], c55br = A.c55[c + nx + 1];
-  // forward strain rates from v(n+1) with the psi of step n
-  T r[4];  // xx = ddxm vx, zz = ddzm vz, zx = ddzp vx, xz = ddxp vz
-  r[0] = tap_m(x1.vx(), c, 1, A.Dx);
-  r[1] = tap_m(x1.vz(), c, nx, A.Dz);
-  r[2] = tap_p(x1.vx(), c, nx, A.Dz);
-  r[3] = tap_p(x1.vz(), c, 1, A.Dx);
-  T ik[4] = {1, 1, 1, 1}, ca[4] = {0, 0, 0, 0}, cb[4] = {0, 0, 0, 0};
-  T *pb[4] = {nullptr, nullptr, nullptr, nullptr};
-  T pbo[4] = {0, 0, 0, 0};
-  const int xs = strip_x(i, nx, A.Lx, A.Rx), zs = strip_z(j, A.nz, A.Tz, A.Bz);
-  if (xs >= 0) {
-    const long long o = (long long)j * A.wx + xs;
-    // x: xx at integer node (PX_VX), xz at half node (PX_VZ)
-    ik[0] = A.tx[T_IK * nx + i]; ca[0] = A.tx[T_A * nx + i]; cb[0] = A.tx[T_B * nx + i];
-    ik[3] = A.tx[T_IKH * nx + i]; ca[3] = A.tx[T_AH * nx + i]; cb[3] = A.tx[T_BH * nx + i];
-    T pn;
-    r[0] = cpml_fwd(r[0], x0.psix()[PX_VX * A.psix_plane + o], ca[0], cb[0], ik[0], &pn);
-    r[3] = cpml_fwd(r[3], x0.psix()[PX_VZ * A.psix_plane + o], ca[3], cb[3], ik[3], &pn);
-    pb[0] = ab.psix() + PX_VX * A.psix_plane + o;
-    pb[3] = ab.psix() + PX_VZ * A.psix_plane + o;
-    pbo[0] = *pb[0];
-    pbo[3] = *pb[3];
+  if (s.z) {
+    cpml_fwd_z(A, s, t.j, (const T *)x0.psiz(), PZ_VZ, T_IK, T_A, T_B, rt[1]);
+    cpml_fwd_z(A, s, t.j, (const T *)x0.psiz(), PZ_VX, T_IKH, T_AH, T_BH, r2);
   }
-  if (zs >= 0) {
-    const int nz = A.nz;
-    const long long o = (long long)zs * nx + i;
-    ik[1] = A.tz[T_IK * nz + j]; ca[1] = A.tz[T_A * nz + j]; cb[1] = A.tz[T_B * nz + j];
-    ik[2] = A.tz[T_IKH * nz + j]; ca[2] = A.tz[T_AH * nz + j]; cb[2] = A.tz[T_BH * nz + j];
-    T pn;
-    r[1] = cpml_fwd(r[1], x0.psiz()[PZ_VZ * A.psiz_plane + o], ca[1], cb[1], ik[1], &pn);
-    r[2] = cpml_fwd(r[2], x0.psiz()[PZ_VX * A.psiz_plane + o], ca[2], cb[2], ik[2], &pn);
-    pb[1] = ab.psiz() + PZ_VZ * A.psiz_plane + o;
-    pb[2] = ab.psiz() + PZ_VX * A.psiz_plane + o;
-    pbo[1] = *pb[1];
-    pbo[2] = *pb[2];
-  }
-  // ---- arithmetic
-  const T rt[3] = {r[0], r[1], r[2] + r[3]};  // xx, zz, engineering xz
-  T S[3] = {0, 0, 0};
+  rt[2] = padd(r2, r3);
+}
+
+// From the effective-rate adjoints eb (times dt) of a group and its memory
+// variables' adjoints mb(q): memory variables (plane 0 at mp), CPML memory,
+// and the strain-rate adjoints rbar.
+template <typename T, int N, typename F>
+__device__ __forceinline__ void adj_memory(const AdjArgs<T> &A, F mb, T *mp, T *pxb, T *pzb, const Strips<T> &s,
+                                           const AdjTile &t, long long c, bool surf, const Pk<T> &tau,
+                                           const Pk<T> (&eb)[3], T *rbar) {
+  const long long np = A.np;
+  Pk<T> rtb[3];
 #pragma unroll
-  for (int n = 0; n < N; ++n)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) S[k] += mo[k * N + n];
-  T e[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) e[k] = N > 0 ? (T(1) + tau) * rt[k] + tau * S[k] : rt[k];
-  const T C13 = c13;
-  const T C11 = A.kind == VI_MEDIUM_ISO ? C13 + T(2) * c55 : c11;
-  const T C33 = A.kind == VI_MEDIUM_ISO ? C11 : c33;
-  const T C55h = T(0.25) * (c55 + c55r + c55b + c55br);
-  const bool surf = A.fs && j == L;
-  const T dt = A.dt;
-  T eb[3];
-  double g11 = g11o, g13 = g13o, g33 = g33o;
-  if (!surf) {
-    eb[0] = dt * (C11 * bxx + C13 * bzz);
-    eb[1] = dt * (C13 * bxx + C33 * bzz);
-    g11 += (double)dt * bxx * e[0];
-    g13 += (double)dt * (bxx * e[1] + bzz * e[0]);
-    g33 += (double)dt * bzz * e[1];
-  } else {
-    // sxx' = sxx + dt (C11 - C13^2/C33) exx; szz' = 0
-    const T ceff = C11 - C13 * C13 / C33;
-    eb[0] = dt * ceff * bxx;
-    eb[1] = T(0);
-    const double w = (double)dt * bxx * e[0];
-    g11 += w;
-    g13 += w * (-2.0 * (double)C13 / (double)C33);
-    g33 += w * ((double)C13 * C13 / ((double)C33 * C33));
-    sbz[c] = T(0);
-  }
-  gc11[c] = g11;
-  gc13[c] = g13;
-  gc33[c] = g33;
-  eb[2] = dt * C55h * bxz;
-  q[c] = dt * bxz * e[2];
-  if (N > 0) {
-    double gt = 0;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) gt += (double)eb[k] * ((double)rt[k] + S[k]);
-    gtau[c] = gto + gt;
-  }
-  // memory variables and the strain-rate adjoints
-  T rtb[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) rtb[k] = (N > 0 ? (T(1) + tau) : T(1)) * eb[k];
+  for (int k = 0; k < 3; ++k) rtb[k] = N > 0 ? pfma(tau, eb[k], eb[k]) : eb[k];
 #pragma unroll
   for (int n = 0; n < N; ++n) {
+    const T e1 = A.dt * A.a1[n], e2 = T(1) + A.dt * A.a2[n];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const bool dead = surf && k == 1;  // Mzz' = 0 on the surface
-      const T mb = dead ? T(0) : mbo[k * N + n];
-      rtb[k] += dt * A.a1[n] * mb;
-      ab.m()[(k * N + n) * np + c] = dead ? T(0) : tau * eb[k] + mb * (T(1) + dt * A.a2[n]);
+      T *q = mp + (k * N + n) * np;
+      if (surf && k == 1) {  // Mzz' = 0 on the surface
+        stvp(q, splat<T>(T(0)), l2_stream());
+      } else {
+        const Pk<T> m = mb(k * N + n);
+        rtb[k] = pfma(splat<T>(e1), m, rtb[k]);
+        stvp(q, pfma(tau, eb[k], pscale(e2, m)), l2_stream());
+      }
     }
   }
-  // psi transposes: rbar = rtbar/kappa + a (psibar' + rtbar), psibar = b (...)
-  T rb[4] = {rtb[0], rtb[1], rtb[2], rtb[2]};
+  Pk<T> rb[4] = {rtb[0], rtb[1], rtb[2], rtb[2]};
+  if (s.x) {
+    cpml_adj_x(A, s, t.gi0, pxb, PX_VX, T_IK, T_A, T_B, rb[0]);
+    cpml_adj_x(A, s, t.gi0, pxb, PX_VZ, T_IKH, T_AH, T_BH, rb[3]);
+  }
+  if (s.z) {
+    cpml_adj_z(A, s, t.j, pzb, PZ_VZ, T_IK, T_A, T_B, rb[1]);
+    cpml_adj_z(A, s, t.j, pzb, PZ_VX, T_IKH, T_AH, T_BH, rb[2]);
+  }
+  if (t.gi0 + VecW<T>::V > A.nx - L)
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (pb[k]) {
-      const T P = pbo[k] + rb[k];
-      *pb[k] = cb[k] * P;
-      rb[k] = rb[k] * ik[k] + ca[k] * P;
-    }
-    rbar[k * np + c] = rb[k];
+    for (int k = 0; k < 4; ++k) zero_outside(rb[k], A.nx - L - t.gi0);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) stvp(rbar + k * np + c, rb[k], bar_policy(A));
+}
+
+// S of a group: the sums of its memory variables
+template <typename T, int N>
+__device__ __forceinline__ void memory_sums(const T *m, long long np, Pk<T> (&S)[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    S[k] = splat<T>(T(0));
+#pragma unroll
+    for (int n = 0; n < N; ++n) S[k] = padd(S[k], ldnp(m + (k * N + n) * np, l2_stream()));
   }
 }
 
+// sigma adjoint and S^T of one step, ISO and VTI.  slot: of the step's start.
+template <typename T, int KIND, int N>
+struct StressK {
+  static constexpr int NACC = KIND == VI_MEDIUM_ISO ? 4 : 5;
+  using S = StressSmem<T, NACC, 3 * N>;
+};
+template <typename T, int KIND, int N>
+__global__ void __launch_bounds__(AdjGeom<T>::NT, N <= 3 ? 2 : 1)
+    k_adj_stress(const __grid_constant__ AdjArgs<T> A, const __grid_constant__ AdjMaps maps, Slot<T> x0, int slot,
+                 int ntx, T *__restrict__ sb, T *__restrict__ mb, T *__restrict__ pxb, T *__restrict__ pzb,
+                 T *__restrict__ rbar, double *__restrict__ acc, int *err) {
+  using G = AdjGeom<T>;
+  using SM = typename StressK<T, KIND, N>::S;
+  constexpr int V = G::V, PL = G::TX * G::TZ;
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
+  auto box = [&](int o) { return reinterpret_cast<T *>(smem + o); };
+  const AdjTile t = adj_tile(A, ntx);
+  const long long ld = A.ld, np = A.np, c = (long long)t.j * ld + t.gi0;
+  if (threadIdx.x == 0) mbar_init(bar, 1);
+  __syncthreads();
+  Pk<T> S[3], tau{}, C11{}, C13{}, C33{};
+  if (t.act) {
+    memory_sums<T, N>((const T *)x0.m() + c, np, S);
+    if (N > 0) tau = ldn(A.tau + c);
+    C13 = ldn(A.c13 + c);
+    if (KIND != VI_MEDIUM_ISO) {
+      C11 = ldn(A.c11 + c);
+      C33 = ldn(A.c33 + c);
+    }
+  }
+  const Strips<T> s = strips_of(A, t.gi0, t.j);
+  if (t.act) prefetch_strips(A, s, t.gi0, t.j, x0, pxb, pzb, PX_VX, PX_VZ, PZ_VZ, PZ_VX);
+  if (threadIdx.x == 0) {
+    mbar_arrive_expect_tx(bar, SM::BYTES);
+    tma_load_4d_hint(box(SM::VX), &maps.st_a, t.x0 - 4, t.z0 - 3, 0, slot + 1, bar, l2_stream());  // new velocities
+    tma_load_4d_hint(box(SM::VZ), &maps.st_a, t.x0 - 4, t.z0 - 4, 1, slot + 1, bar, l2_stream());
+    tma_load_2d(box(SM::CC), &maps.cc, t.x0, t.z0, bar);
+    tma_load_3d(box(SM::SB), &maps.own, t.x0, t.z0, 0, bar);
+    if (N > 0) tma_load_3d_hint(box(SM::MB), &maps.mem, t.x0, t.z0, 0, bar, l2_stream());
+    tma_load_3d_hint(smem + SM::ACC, &maps.acc, t.x0, t.z0, 0, bar, l2_stream());
+    pdl_wait();  // dbar: the previous kernel's
+    tma_load_3d_hint(box(SM::D0), &maps.px, t.x0 - 4, t.z0, 0, bar, bar_policy(A));
+    tma_load_3d_hint(box(SM::D1), &maps.pz, t.x0, t.z0 - 3, 1, bar, bar_policy(A));
+    tma_load_3d_hint(box(SM::D2), &maps.px, t.x0 - 4, t.z0, 2, bar, bar_policy(A));
+    tma_load_3d_hint(box(SM::D3), &maps.pz, t.x0, t.z0 - 4, 3, bar, bar_policy(A));
+  }
+  pdl_wait();  // every thread, before its first store
+  pdl_release();
+  if (!boxes_landed(bar, err) || !t.act) return;
+  const bool surf = A.fs && t.j == L;
+  const int ow = t.r * G::WX + t.lx + 4, oz = t.r * G::TX + t.lx, oc = t.r * G::WC + t.lx;
+  Pk<T> bxx, bzz, bxz;
+  adj_sigma(A, t, box(SM::SB) + oz, box(SM::D0) + ow, box(SM::D1) + oz + 3 * G::TX, box(SM::D2) + ow,
+            box(SM::D3) + oz + 4 * G::TX, bxx, bzz, bxz);
+  stv(sb + c, bxx);
+  stv(sb + np + c, surf ? splat<T>(T(0)) : bzz);  // szz' = 0 on the surface
+  stv(sb + 2 * np + c, bxz);
+  Pk<T> rt[3], e[3];
+  adj_rates(A, x0, s, t, box(SM::VX) + ow + 3 * G::WX, box(SM::VZ) + ow + 4 * G::WX, rt);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) e[k] = N > 0 ? pfma(tau, padd(rt[k], S[k]), rt[k]) : rt[k];
+  const T *cc = box(SM::CC) + oc;
+  const Pk<T> c55 = ldv(cc), c55d = ldv(cc + G::WC);
+  Pk<T> C55h;
+#pragma unroll
+  for (int k = 0; k < V; ++k)
+    C55h.v[k] = T(0.25) * (c55.v[k] + right_of(c55, k, cc[V]) + c55d.v[k] + right_of(c55d, k, cc[G::WC + V]));
+  if (KIND == VI_MEDIUM_ISO) C11 = C33 = pfma(splat<T>(T(2)), c55, C13);
+  // accumulators: plane 0 TAU, 1 Q55, 2 C11 (ISO: C11 and C33), 3 C13, 4 C33
+  const double *ai = reinterpret_cast<const double *>(smem + SM::ACC) + oz;
+  double *ao = acc + c;
+  Pk<T> eb[3];
+  if (!surf) {
+    eb[0] = pscale(A.dt, pfma(C11, bxx, pmul(C13, bzz)));
+    eb[1] = pscale(A.dt, pfma(C13, bxx, pmul(C33, bzz)));
+    if (KIND == VI_MEDIUM_ISO) {
+      acc_add<T>(ai + 2 * PL, ao + 2 * np, [&](int k, double g) {
+        return fma((double)bxx.v[k], (double)e[0].v[k], fma((double)bzz.v[k], (double)e[1].v[k], g));
+      });
+    } else {
+      acc_add<T>(ai + 2 * PL, ao + 2 * np, [&](int k, double g) { return fma((double)bxx.v[k], (double)e[0].v[k], g); });
+      acc_add<T>(ai + 4 * PL, ao + 4 * np, [&](int k, double g) { return fma((double)bzz.v[k], (double)e[1].v[k], g); });
+    }
+    acc_add<T>(ai + 3 * PL, ao + 3 * np, [&](int k, double g) {
+      return fma((double)bxx.v[k], (double)e[1].v[k], fma((double)bzz.v[k], (double)e[0].v[k], g));
+    });
+  } else {
+    // sxx' = sxx + dt (C11 - C13^2/C33) exx
+#pragma unroll
+    for (int k = 0; k < V; ++k) eb[0].v[k] = A.dt * (C11.v[k] - C13.v[k] * C13.v[k] / C33.v[k]) * bxx.v[k];
+    eb[1] = splat<T>(T(0));
+    auto w = [&](int k) { return (double)bxx.v[k] * (double)e[0].v[k]; };
+    auto f = [&](int k) { return (double)C13.v[k] / (double)C33.v[k]; };
+    if (KIND == VI_MEDIUM_ISO) {
+      acc_add<T>(ai + 2 * PL, ao + 2 * np, [&](int k, double g) { return g + w(k) * (1.0 + f(k) * f(k)); });
+    } else {
+      acc_add<T>(ai + 2 * PL, ao + 2 * np, [&](int k, double g) { return g + w(k); });
+      acc_add<T>(ai + 4 * PL, ao + 4 * np, [&](int k, double g) { return g + w(k) * (f(k) * f(k)); });
+    }
+    acc_add<T>(ai + 3 * PL, ao + 3 * np, [&](int k, double g) { return g - 2.0 * w(k) * f(k); });
+  }
+  eb[2] = pscale(A.dt, pmul(C55h, bxz));
+  acc_add<T>(ai + PL, ao + np, [&](int k, double g) { return fma((double)bxz.v[k], (double)e[2].v[k], g); });
+  if (N > 0)
+    acc_add<T>(ai, ao, [&](int k, double g) {
+      double u = (double)eb[0].v[k] * ((double)rt[0].v[k] + (double)S[0].v[k]);
+      u = fma((double)eb[1].v[k], (double)rt[1].v[k] + (double)S[1].v[k], u);
+      return g + fma((double)eb[2].v[k], (double)rt[2].v[k] + (double)S[2].v[k], u);
+    });
+  const T *ms = box(SM::MB) + oz;
+  adj_memory<T, N>(A, [&](int q) { return ldv(ms + q * PL); }, mb + c, pxb, pzb, s, t, c, surf, tau, eb, rbar);
+}
 
-// ---- S^T for TTI media --------------------------------------------------
+// v += -D^T rbar, the residual at the receivers of step it, and V^T of the
+// velocity stage: dbar (4 planes: sxx-x, sxz-z, sxz-x, szz-z) and the
+// buoyancy terms d(vx')/d rho = dt (-bx^2 / 2) (div + f), likewise vz.
+template <typename T>
+__global__ void __launch_bounds__(AdjGeom<T>::NT, 5)
+    k_adj_vel(const __grid_constant__ AdjArgs<T> A, const __grid_constant__ AdjMaps maps, Slot<T> x0, Slot<T> x1,
+              int slot, const __grid_constant__ FusedExtras<T> x, const T *obs, T *__restrict__ vb,
+              T *__restrict__ pxb, T *__restrict__ pzb, T *__restrict__ dbar, double *__restrict__ acc) {
+  using G = AdjGeom<T>;
+  using SM = VelSmem<T>;
+  constexpr int V = G::V, PL = G::TX * G::TZ;
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
+  auto box = [&](int o) { return reinterpret_cast<T *>(smem + o); };
+  const AdjTile t = adj_tile(A, x.ntx);
+  const long long ld = A.ld, np = A.np, c = (long long)t.j * ld + t.gi0;
+  if (threadIdx.x == 0) mbar_init(bar, 1);
+  __syncthreads();
+  Pk<T> r0{}, r1{};
+  T rr = 0;
+  if (t.act) {
+    r0 = ldn(A.rho + c);
+    r1 = ldn(A.rho + c + ld);
+    rr = ldn1(A.rho + c + V);
+  }
+  const Strips<T> s = strips_of(A, t.gi0, t.j);
+  if (t.act) prefetch_strips(A, s, t.gi0, t.j, x0, pxb, pzb, PX_SXX, PX_SXZ, PZ_SXZ, PZ_SZZ);
+  if (threadIdx.x == 0) {
+    mbar_arrive_expect_tx(bar, SM::BYTES);
+    tma_load_4d_hint(box(SM::SXX), &maps.st_a, t.x0 - 4, t.z0, 2, slot, bar, l2_stream());
+    tma_load_4d_hint(box(SM::SXZ), &maps.st_b, t.x0 - 4, t.z0 - 4, 4, slot, bar, l2_stream());
+    tma_load_4d_hint(box(SM::SZZ), &maps.st_c, t.x0, t.z0 - 3, 3, slot, bar, l2_stream());
+    tma_load_3d(box(SM::VB), &maps.own, t.x0, t.z0, 0, bar);
+    tma_load_3d_hint(smem + SM::ACC, &maps.acc, t.x0, t.z0, 0, bar, l2_stream());
+    pdl_wait();  // rbar: the previous kernel's
+    tma_load_3d_hint(box(SM::R0), &maps.px, t.x0 - 4, t.z0, 0, bar, bar_policy(A));
+    tma_load_3d_hint(box(SM::R1), &maps.pz, t.x0, t.z0 - 3, 1, bar, bar_policy(A));
+    tma_load_3d_hint(box(SM::R2), &maps.pz, t.x0, t.z0 - 4, 2, bar, bar_policy(A));
+    tma_load_3d_hint(box(SM::R3), &maps.px, t.x0 - 4, t.z0, 3, bar, bar_policy(A));
+  }
+  const int e0 = x.tile_off[blockIdx.x], e1 = x.tile_off[blockIdx.x + 1];
+  pdl_wait();
+  pdl_release();
+  if (!boxes_landed(bar, x.err)) return;
+  const int ow = t.r * G::WX + t.lx + 4, oz = t.r * G::TX + t.lx;
+  if (e0 < e1) {  // a tile with entries: its residuals into the staged v adjoint, one thread per receiver
+    T *sv = box(SM::VB);
+    for (int e = e0 + (int)threadIdx.x; e < e1; e += G::NT) {
+      const int4 en = x.tile_ent[e];
+      if (en.w != TL_RECEIVER) continue;
+      const long long r = (long long)en.y * ld + en.x;
+      const int o = (en.y - t.z0) * G::TX + en.x - t.x0;
+      atomicAdd(sv + o, x1.vx()[r] - obs[(long long)en.z * x.tnt + x.it]);
+      atomicAdd(sv + PL + o, x1.vz()[r] - obs[(long long)(x.nrec + en.z) * x.tnt + x.it]);
+    }
+    __syncthreads();
+  }
+  if (!t.act) return;
+  Pk<T> vx = psub(ldv(box(SM::VB) + oz),
+                  padd(dxp(ldwin(box(SM::R0) + ow), A.Dx), dzm(box(SM::R2) + oz + 4 * G::TX, G::TX, A.Dz)));
+  Pk<T> vz = psub(ldv(box(SM::VB) + PL + oz),
+                  padd(dzp(box(SM::R1) + oz + 3 * G::TX, G::TX, A.Dz), dxm(ldwin(box(SM::R3) + ow), A.Dx)));
+  if (t.gi0 + V > A.nx - L) {
+    zero_outside(vx, A.nx - L - t.gi0);
+    zero_outside(vz, A.nx - L - t.gi0);
+  }
+  stv(vb + c, vx);
+  stv(vb + np + c, vz);
+  // forward stress divergence of the step
+  const T *sq = box(SM::SXZ) + ow + 4 * G::WX;
+  Pk<T> d0 = dxp(ldwin(box(SM::SXX) + ow), A.Dx), d2 = dxm(ldwin(sq), A.Dx);
+  Pk<T> d1 = dzm(sq, G::WX, A.Dz), d3 = dzp(box(SM::SZZ) + oz + 3 * G::TX, G::TX, A.Dz);
+  if (s.x) {
+    cpml_fwd_x(A, s, t.gi0, (const T *)x0.psix(), PX_SXX, T_IKH, T_AH, T_BH, d0);
+    cpml_fwd_x(A, s, t.gi0, (const T *)x0.psix(), PX_SXZ, T_IK, T_A, T_B, d2);
+  }
+  if (s.z) {
+    cpml_fwd_z(A, s, t.j, (const T *)x0.psiz(), PZ_SXZ, T_IK, T_A, T_B, d1);
+    cpml_fwd_z(A, s, t.j, (const T *)x0.psiz(), PZ_SZZ, T_IKH, T_AH, T_BH, d3);
+  }
+  Pk<T> dx = padd(d0, d1), dz = padd(d2, d3), bx, bz;
+#pragma unroll
+  for (int k = 0; k < V; ++k) {
+    bx.v[k] = T(2) / (r0.v[k] + right_of(r0, k, rr));
+    bz.v[k] = T(2) / (r0.v[k] + r1.v[k]);
+  }
+  for (int e = e0; e < e1; ++e) {  // force sources: their buoyancy factor depends on rho too
+    const int4 en = x.tile_ent[e];
+    if (en.w > TL_FORCE_Z) break;
+    if (en.y != t.j || en.x < t.gi0 || en.x >= t.gi0 + V) continue;
+    const T f = x.it < x.wnt ? x.amp[en.z] * x.wavelet[(long long)en.z * x.wnt + x.it] : T(0);
+#pragma unroll
+    for (int k = 0; k < V; ++k)
+      if (k == en.x - t.gi0) (en.w == TL_FORCE_X ? dx.v[k] : dz.v[k]) += f;
+  }
+  const Pk<T> hx = pmul(pmul(pscale(A.dt * T(-0.5), pmul(bx, bx)), dx), vx);
+  const Pk<T> hz = pmul(pmul(pscale(A.dt * T(-0.5), pmul(bz, bz)), dz), vz);
+  const double *ai = reinterpret_cast<const double *>(smem + SM::ACC) + oz;
+  acc_add<T>(ai, acc + c, [&](int k, double g) { return g + (double)hx.v[k]; });
+  acc_add<T>(ai + PL, acc + np + c, [&](int k, double g) { return g + (double)hz.v[k]; });
+  Pk<T> db[4];
+  db[0] = db[1] = pmul(pscale(A.dt, bx), vx);
+  db[2] = db[3] = pmul(pscale(A.dt, bz), vz);
+  if (s.x) {
+    cpml_adj_x(A, s, t.gi0, pxb, PX_SXX, T_IKH, T_AH, T_BH, db[0]);
+    cpml_adj_x(A, s, t.gi0, pxb, PX_SXZ, T_IK, T_A, T_B, db[2]);
+  }
+  if (s.z) {
+    cpml_adj_z(A, s, t.j, pzb, PZ_SXZ, T_IK, T_A, T_B, db[1]);
+    cpml_adj_z(A, s, t.j, pzb, PZ_SZZ, T_IKH, T_AH, T_BH, db[3]);
+  }
+  if (t.gi0 + V > A.nx - L)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) zero_outside(db[k], A.nx - L - t.gi0);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) stvp(dbar + k * np + c, db[k], bar_policy(A));
+}
+
+// ---- TTI ----------------------------------------------------------------
 // The TTI stress law couples neighbouring cells (custom_solver/Model.jl:59-108
 // on the staggered grid):
 //   dsxx = C11 exx + C13 ezz + C15 ebxz,   dszz = C13 exx + C33 ezz + C35 ebxz,
@@ -310,491 +886,320 @@ __global__ void __launch_bounds__(256) k_stress_t(AdjArgs<T> A, Slot<T> x0, Slot
 // ebzz the means of exx, ezz over (i,j),(i+1,j),(i,j+1),(i+1,j+1), C15h,
 // C35h, C55h the means of the stiffness over the latter four cells, and on
 // the free surface (row L) ezz = -(C13 exx + C35 ebxz) / C33.  Effective
-// rates outside the update region U are zero.  The transpose runs in four
-// kernels: the forward rates (k_tti_fwd_rates, k_tti_fwd_surface), the
-// effective-rate adjoints gathered from the stress adjoints
-// (k_tti_ebar_t), the surface relation transposed (k_tti_surface_t) and the
-// per-cell rest — memory variables, tau, CPML psi (k_tti_stress_t).  Every
-// cell gathers its own terms: no atomics.
-template <typename T>
-__device__ __forceinline__ bool in_u(int i, int j, int nx, int nz) {
-  return i >= L && i < nx - L && j >= L && j < nz - L;
-}
+// rates and stress adjoints outside the update region are zero.
 
-// Forward effective rates e (3 planes) and rt + S (3 planes: the CPML'd
-// strain rates plus the memory-variable sums, de/dtau) of step it, from the
-// new velocities (x1) and the CPML memory and memory variables before the
-// step (x0).  fe is zero outside U.
+// sigma adjoint of the step, and its forward effective rates: fe holds e (3
+// planes, ezz on the surface row before the surface relation) and rt + S (3
+// planes: the strain rates plus the memory-variable sums, de/dtau).
+template <typename T>
+struct SigmaTtiSmem {
+  using S = StressSmem<T, 0, 0>;
+  static constexpr int SIZE = S::CC;  // the boxes up to the sigma adjoint
+  static constexpr int BYTES = S::TAPS + S::VBOX + 3 * AdjGeom<T>::TX * AdjGeom<T>::TZ * AdjGeom<T>::E;
+};
 template <typename T, int N>
-__global__ void __launch_bounds__(256) k_tti_fwd_rates(AdjArgs<T> A, Slot<T> x0, Slot<T> x1, T *fe) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + L;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + L;
-  if (i >= A.nx - L || j >= A.nz - L) return;
-  const int nx = A.nx;
-  const long long c = (long long)j * nx + i, np = A.np;
-  T r[4];
-  r[0] = tap_m(x1.vx(), c, 1, A.Dx);
-  r[1] = tap_m(x1.vz(), c, nx, A.Dz);
-  r[2] = tap_p(x1.vx(), c, nx, A.Dz);
-  r[3] = tap_p(x1.vz(), c, 1, A.Dx);
-  const int xs = strip_x(i, nx, A.Lx, A.Rx), zs = strip_z(j, A.nz, A.Tz, A.Bz);
-  T pn;
-  if (xs >= 0) {
-    const long long o = (long long)j * A.wx + xs;
-    r[0] = cpml_fwd(r[0], x0.psix()[PX_VX * A.psix_plane + o], A.tx[T_A * nx + i], A.tx[T_B * nx + i],
-                    A.tx[T_IK * nx + i], &pn);
-    r[3] = cpml_fwd(r[3], x0.psix()[PX_VZ * A.psix_plane + o], A.tx[T_AH * nx + i], A.tx[T_BH * nx + i],
-                    A.tx[T_IKH * nx + i], &pn);
+__global__ void __launch_bounds__(AdjGeom<T>::NT, 4)
+    k_adj_sigma_tti(const __grid_constant__ AdjArgs<T> A, const __grid_constant__ AdjMaps maps, Slot<T> x0, int slot,
+                    int ntx, T *__restrict__ sb, T *__restrict__ fe, int *err) {
+  using G = AdjGeom<T>;
+  using SM = typename SigmaTtiSmem<T>::S;
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
+  auto box = [&](int o) { return reinterpret_cast<T *>(smem + o); };
+  const AdjTile t = adj_tile(A, ntx);
+  const long long ld = A.ld, np = A.np, c = (long long)t.j * ld + t.gi0;
+  if (threadIdx.x == 0) mbar_init(bar, 1);
+  __syncthreads();
+  Pk<T> S[3], tau{};
+  if (t.act) {
+    memory_sums<T, N>((const T *)x0.m() + c, np, S);
+    if (N > 0) tau = ldn(A.tau + c);
   }
-  if (zs >= 0) {
-    const int nz = A.nz;
-    const long long o = (long long)zs * nx + i;
-    r[1] = cpml_fwd(r[1], x0.psiz()[PZ_VZ * A.psiz_plane + o], A.tz[T_A * nz + j], A.tz[T_B * nz + j],
-                    A.tz[T_IK * nz + j], &pn);
-    r[2] = cpml_fwd(r[2], x0.psiz()[PZ_VX * A.psiz_plane + o], A.tz[T_AH * nz + j], A.tz[T_BH * nz + j],
-                    A.tz[T_IKH * nz + j], &pn);
+  if (threadIdx.x == 0) {
+    mbar_arrive_expect_tx(bar, SigmaTtiSmem<T>::BYTES);
+    tma_load_4d_hint(box(SM::VX), &maps.st_a, t.x0 - 4, t.z0 - 3, 0, slot + 1, bar, l2_stream());
+    tma_load_4d_hint(box(SM::VZ), &maps.st_a, t.x0 - 4, t.z0 - 4, 1, slot + 1, bar, l2_stream());
+    tma_load_3d(box(SM::SB), &maps.own, t.x0, t.z0, 0, bar);
+    pdl_wait();  // dbar: the previous kernel's
+    tma_load_3d_hint(box(SM::D0), &maps.px, t.x0 - 4, t.z0, 0, bar, bar_policy(A));
+    tma_load_3d_hint(box(SM::D1), &maps.pz, t.x0, t.z0 - 3, 1, bar, bar_policy(A));
+    tma_load_3d_hint(box(SM::D2), &maps.px, t.x0 - 4, t.z0, 2, bar, bar_policy(A));
+    tma_load_3d_hint(box(SM::D3), &maps.pz, t.x0, t.z0 - 4, 3, bar, bar_policy(A));
   }
-  const T rt[3] = {r[0], r[1], r[2] + r[3]};
-  T S[3] = {0, 0, 0};
-#pragma unroll
-  for (int n = 0; n < N; ++n)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) S[k] += x0.m()[(k * N + n) * np + c];
-  const T tau = N > 0 ? A.tau[c] : T(0);
+  pdl_wait();
+  pdl_release();
+  if (!boxes_landed(bar, err) || !t.act) return;
+  const int ow = t.r * G::WX + t.lx + 4, oz = t.r * G::TX + t.lx;
+  Pk<T> bxx, bzz, bxz;
+  adj_sigma(A, t, box(SM::SB) + oz, box(SM::D0) + ow, box(SM::D1) + oz + 3 * G::TX, box(SM::D2) + ow,
+            box(SM::D3) + oz + 4 * G::TX, bxx, bzz, bxz);
+  stv(sb + c, bxx);
+  stv(sb + np + c, A.fs && t.j == L ? splat<T>(T(0)) : bzz);  // szz' = 0 on the surface
+  stv(sb + 2 * np + c, bxz);
+  const Strips<T> s = strips_of(A, t.gi0, t.j);
+  Pk<T> rt[3];
+  adj_rates(A, x0, s, t, box(SM::VX) + ow + 3 * G::WX, box(SM::VZ) + ow + 4 * G::WX, rt);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    fe[k * np + c] = N > 0 ? (T(1) + tau) * rt[k] + tau * S[k] : rt[k];
-    fe[(3 + k) * np + c] = rt[k] + S[k];
+    const Pk<T> rs = padd(rt[k], S[k]);
+    Pk<T> e = N > 0 ? pfma(tau, rs, rt[k]) : rt[k];
+    if (t.gi0 + G::V > A.nx - L) zero_outside(e, A.nx - L - t.gi0);
+    stv(fe + k * np + c, e);
+    stv(fe + (3 + k) * np + c, rs);
   }
 }
 
-// The free-surface relation of the forward step on row L:
-// ezz = -(C13 exx + C35 ebxz) / C33 (row L - 1 lies outside U: zero there).
+// u[-1 .. V] of a row
 template <typename T>
-__global__ void k_tti_fwd_surface(AdjArgs<T> A, T *fe) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + L;
-  if (i >= A.nx - L) return;
-  const int nx = A.nx;
-  const long long np = A.np, c = (long long)L * nx + i;
-  const T *exx = fe, *exz = fe + 2 * np;
-  const T eb = T(0.25) * (exz[c] + exz[c - 1] + exz[c - nx] + exz[c - nx - 1]);
-  fe[np + c] = -(A.c13[c] * exx[c] + A.c35[c] * eb) / A.c33[c];
+struct Row3 {
+  T w[VecW<T>::V + 2];
+};
+template <typename T>
+__device__ __forceinline__ Row3<T> ldrow3(const T *u) {
+  constexpr int V = VecW<T>::V;
+  Row3<T> r;
+  const Pk<T> t = ldv(u);
+  r.w[0] = u[-1];
+  r.w[V + 1] = u[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) r.w[1 + k] = t.v[k];
+  return r;
+}
+// mean of the four cells (i, j), (i+1, j), (i, j+1), (i+1, j+1), cell o - 1 of
+// the group (o = 0: the cell before it)
+template <typename T>
+__device__ __forceinline__ T mean_of(const Row3<T> &a, const Row3<T> &b, int o) {
+  return T(0.25) * (a.w[o] + a.w[o + 1] + b.w[o] + b.w[o + 1]);
 }
 
-// Adjoints of the effective rates (3 planes eb) gathered from the stress
-// adjoints of the cells whose update reads them, and the direct stiffness
-// gradient terms: C11, C13, C33, C15 and C35 at the cell, and the
-// per-cell products q (C55h), q15 (C15h), q35 (C35h) that k_gather and
-// k_tti_gather spread over the four cells of each half-node mean.  On the
-// free surface the stress szz is reset after the update, so its adjoint
-// there is zero.
-template <typename T>
-__global__ void __launch_bounds__(256) k_tti_ebar_t(AdjArgs<T> A, Slot<T> ab, const T *fe, T *eb, T *q,
-                                                     T *q15, T *q35, double *g11, double *g13, double *g15,
-                                                     double *g33, double *g35) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + L;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + L;
-  const int nx = A.nx, nz = A.nz;
-  if (i >= nx - L || j >= nz - L) return;
-  const long long c = (long long)j * nx + i, np = A.np;
-  const T *sbx = ab.sxx(), *sbz = ab.szz(), *sbq = ab.sxz();
-  const T *exx = fe, *ezz = fe + np, *exz = fe + 2 * np;
-  const T dt = A.dt;
-  auto bzz = [&](int ii, int jj) -> T {  // szz adjoint of a cell of U (zero on the surface)
-    return (A.fs && jj == L) ? T(0) : sbz[(long long)jj * nx + ii];
-  };
-  auto mean4p = [&](const T *u, long long cc) { return T(0.25) * (u[cc] + u[cc + 1] + u[cc + nx] + u[cc + nx + 1]); };
-  const T bxx = sbx[c], bzc = bzz(i, j), bxz = sbq[c];
-  const T C11 = A.c11[c], C13 = A.c13[c], C33 = A.c33[c], C15 = A.c15[c], C35 = A.c35[c];
-  const T C55h = mean4p(A.c55, c);
-  // exz feeds sxx, szz of the cells (i,j), (i+1,j), (i,j+1), (i+1,j+1)
-  T sq = 0;
-#pragma unroll
-  for (int dj = 0; dj <= 1; ++dj)
-#pragma unroll
-    for (int di = 0; di <= 1; ++di) {
-      const int ii = i + di, jj = j + dj;
-      if (in_u<T>(ii, jj, nx, nz)) {
-        const long long cc = (long long)jj * nx + ii;
-        sq += A.c15[cc] * sbx[cc] + A.c35[cc] * bzz(ii, jj);
-      }
-    }
-  // exx, ezz feed sxz of the cells (i,j), (i-1,j), (i,j-1), (i-1,j-1)
-  T sx = 0, sz = 0;
-#pragma unroll
-  for (int dj = 0; dj <= 1; ++dj)
-#pragma unroll
-    for (int di = 0; di <= 1; ++di) {
-      const int ii = i - di, jj = j - dj;
-      if (in_u<T>(ii, jj, nx, nz)) {
-        const long long cc = (long long)jj * nx + ii;
-        sx += mean4p(A.c15, cc) * sbq[cc];
-        sz += mean4p(A.c35, cc) * sbq[cc];
-      }
-    }
-  eb[c] = dt * (C11 * bxx + C13 * bzc + T(0.25) * sx);
-  eb[np + c] = dt * (C13 * bxx + C33 * bzc + T(0.25) * sz);
-  eb[2 * np + c] = dt * (C55h * bxz + T(0.25) * sq);
-  // forward rates at the cell and the neighbour means its update used
-  const T ex = exx[c], ez = ezz[c], eq = exz[c];
-  const T ebxz = T(0.25) * (exz[c] + exz[c - 1] + exz[c - nx] + exz[c - nx - 1]);
-  const T ebxx = mean4p(exx, c), ebzz = mean4p(ezz, c);
-  g11[c] += (double)dt * bxx * ex;
-  g13[c] += (double)dt * ((double)bxx * ez + (double)bzc * ex);
-  g33[c] += (double)dt * bzc * ez;
-  g15[c] += (double)dt * bxx * ebxz;
-  g35[c] += (double)dt * bzc * ebxz;
-  q[c] = dt * bxz * eq;
-  q15[c] = dt * bxz * ebxx;
-  q35[c] = dt * bxz * ebzz;
-}
-
-// The surface relation transposed (row L): the adjoint of the surface ezz
-// (as k_tti_ebar_t gathered it) moves to exx of the cell and to exz of the
-// cell and its left neighbour, and adds its stiffness terms; the surface
-// ezz adjoint itself is read as zero afterwards (k_tti_stress_t).
-template <typename T>
-__global__ void k_tti_surface_t(AdjArgs<T> A, const T *fe, T *eb, double *g13, double *g33, double *g35) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + L;
-  const int nx = A.nx;
-  if (i >= nx - L) return;
-  const long long np = A.np, c = (long long)L * nx + i;
-  const T *exx = fe, *ezz = fe + np, *exz = fe + 2 * np;
-  const T zb = eb[np + c];
-  const T C33 = A.c33[c];
-  eb[c] += -A.c13[c] / C33 * zb;
-  T xz = -T(0.25) * A.c35[c] / C33 * zb;
-  if (i + 1 < nx - L) xz -= T(0.25) * A.c35[c + 1] / A.c33[c + 1] * eb[np + c + 1];
-  eb[2 * np + c] += xz;
-  const T ebs = T(0.25) * (exz[c] + exz[c - 1] + exz[c - nx] + exz[c - nx - 1]);
-  g13[c] += -(double)zb * exx[c] / C33;
-  g35[c] += -(double)zb * ebs / C33;
-  g33[c] += -(double)zb * ezz[c] / C33;
-}
-
-// Memory variables, the tau gradient and the CPML psi transposes of a TTI
-// cell, from the effective-rate adjoints: rbar (4 planes) as k_stress_t
-// leaves it.
+// S^T of one TTI step: the effective-rate adjoints gathered from the stress
+// adjoints of the cells whose update reads them, the stiffness terms, the
+// surface relation transposed, then memory variables, tau and CPML memory.
 template <typename T, int N>
-__global__ void __launch_bounds__(256) k_tti_stress_t(AdjArgs<T> A, Slot<T> ab, const T *fe, const T *eb,
-                                                       T *rbar, double *gtau) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + L;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + L;
-  const int nx = A.nx;
-  if (i >= nx - L || j >= A.nz - L) return;
-  const long long c = (long long)j * nx + i, np = A.np;
-  const bool surf = A.fs && j == L;
-  T e_b[3] = {eb[c], surf ? T(0) : eb[np + c], eb[2 * np + c]};
-  if (surf) ab.szz()[c] = T(0);
-  const T tau = N > 0 ? A.tau[c] : T(0);
-  if (N > 0) {
-    double gt = 0;
+__global__ void __launch_bounds__(AdjGeom<T>::NT, 3)
+    k_adj_stress_tti(const __grid_constant__ AdjArgs<T> A, const __grid_constant__ AdjMaps maps, int ntx, const T *fe,
+                     T *__restrict__ mbar, T *__restrict__ pxb, T *__restrict__ pzb, T *__restrict__ rbar,
+                     double *__restrict__ acc, int *err) {
+  using G = AdjGeom<T>;
+  using SM = TtiSmem<T>;
+  constexpr int V = G::V, PL = G::TX * G::TZ, W = G::WX, RP = G::WX * SM::RH, NM = N > 0 ? 3 * N : 1;
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
+  auto box = [&](int o) { return reinterpret_cast<T *>(smem + o); };
+  const AdjTile t = adj_tile(A, ntx);
+  const long long ld = A.ld, np = A.np, c = (long long)t.j * ld + t.gi0;
+  if (threadIdx.x == 0) mbar_init(bar, 1);
+  __syncthreads();
+  Pk<T> C11{}, C13{}, C33{}, tau{}, mb[NM];
+  if (t.act) {
+    C11 = ldn(A.c11 + c);
+    C13 = ldn(A.c13 + c);
+    C33 = ldn(A.c33 + c);
+    if (N > 0) tau = ldn(A.tau + c);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) gt += (double)e_b[k] * fe[(3 + k) * np + c];
-    gtau[c] += gt;
+    for (int q = 0; q < 3 * N; ++q) mb[q] = ldcgv(mbar + q * np + c);
   }
-  T rtb[3];
+  if (threadIdx.x == 0) {
+    mbar_arrive_expect_tx(bar, SM::BYTES);
+    tma_load_2d(box(SM::C15), &maps.c2, t.x0 - 4, t.z0 - 1, bar);
+    tma_load_2d(box(SM::C35), &maps.c3, t.x0 - 4, t.z0 - 1, bar);
+    tma_load_2d(box(SM::CC), &maps.cc, t.x0, t.z0, bar);
+    tma_load_3d_hint(smem + SM::ACC, &maps.acc, t.x0, t.z0, 0, bar, l2_stream());
+    pdl_wait();  // sigma adjoint and effective rates: the previous kernel's
+    tma_load_3d(box(SM::FE), &maps.px, t.x0 - 4, t.z0 - 1, 0, bar);
+    tma_load_3d(box(SM::SB), &maps.pz, t.x0 - 4, t.z0 - 1, 0, bar);
+  }
+  pdl_wait();
+  pdl_release();
+  Pk<T> rs[3];
+  if (N > 0 && t.act)
 #pragma unroll
-  for (int k = 0; k < 3; ++k) rtb[k] = (N > 0 ? (T(1) + tau) : T(1)) * e_b[k];
+    for (int k = 0; k < 3; ++k) rs[k] = ldcgv(fe + (3 + k) * np + c);
+  if (!boxes_landed(bar, err) || !t.act) return;
+  const bool surf = A.fs && t.j == L;
+  const int o = (t.r + 1) * W + t.lx + 4, oc = t.r * G::WC + t.lx, oz = t.r * G::TX + t.lx;
+  const T *f0 = box(SM::FE) + o, *b0 = box(SM::SB) + o;
+  const double *ai = reinterpret_cast<const double *>(smem + SM::ACC) + oz;
+  double *ao = acc + c;
+  Pk<T> eb[3], exx, ezz, exz, ebxz, bxz, c35own;  // eb without dt until the end
+  const Pk<T> bxx = ldv(b0), bzz = ldv(b0 + RP);
+  eb[0] = pfma(C11, bxx, pmul(C13, bzz));
+  eb[1] = pfma(C13, bxx, pmul(C33, bzz));
+  // the zz effective-rate adjoint of the cell after the group (surface row)
+  T zr = 0, wr = 0;
+  if (surf && t.gi0 + V < A.nx - L) {
+    const T *q = b0 + 2 * RP + V, *a = box(SM::C35) + o + V;
+    T sz = 0;
 #pragma unroll
-  for (int n = 0; n < N; ++n) {
+    for (int di = 0; di <= 1; ++di)  // row L - 1 lies outside the update region
+      sz += T(0.25) * (a[-di] + a[1 - di] + a[W - di] + a[W + 1 - di]) * q[-di];
+    zr = ldn1(A.c13 + c + V) * b0[V] + T(0.25) * sz;
+    wr = a[0] / ldn1(A.c33 + c + V);
+  }
+  {  // exx, ezz feed sxz of the cells (i,j), (i-1,j), (i,j-1), (i-1,j-1)
+    const Row3<T> q0 = ldrow3(b0 + 2 * RP), qm = ldrow3(b0 + 2 * RP - W);
+    {
+      const T *cc = box(SM::CC) + oc;
+      const Pk<T> c55 = ldv(cc), c55d = ldv(cc + G::WC);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const bool dead = surf && k == 1;  // Mzz' = 0 on the surface
-      T *mp = ab.m() + (k * N + n) * np + c;
-      const T mb = dead ? T(0) : *mp;
-      rtb[k] += A.dt * A.a1[n] * mb;
-      *mp = dead ? T(0) : tau * e_b[k] + mb * (T(1) + A.dt * A.a2[n]);
-    }
-  }
-  T ik[4] = {1, 1, 1, 1}, ca[4] = {0, 0, 0, 0}, cb[4] = {0, 0, 0, 0};
-  T *pb[4] = {nullptr, nullptr, nullptr, nullptr};
-  const int xs = strip_x(i, nx, A.Lx, A.Rx), zs = strip_z(j, A.nz, A.Tz, A.Bz);
-  if (xs >= 0) {
-    const long long o = (long long)j * A.wx + xs;
-    ik[0] = A.tx[T_IK * nx + i]; ca[0] = A.tx[T_A * nx + i]; cb[0] = A.tx[T_B * nx + i];
-    ik[3] = A.tx[T_IKH * nx + i]; ca[3] = A.tx[T_AH * nx + i]; cb[3] = A.tx[T_BH * nx + i];
-    pb[0] = ab.psix() + PX_VX * A.psix_plane + o;
-    pb[3] = ab.psix() + PX_VZ * A.psix_plane + o;
-  }
-  if (zs >= 0) {
-    const int nz = A.nz;
-    const long long o = (long long)zs * nx + i;
-    ik[1] = A.tz[T_IK * nz + j]; ca[1] = A.tz[T_A * nz + j]; cb[1] = A.tz[T_B * nz + j];
-    ik[2] = A.tz[T_IKH * nz + j]; ca[2] = A.tz[T_AH * nz + j]; cb[2] = A.tz[T_BH * nz + j];
-    pb[1] = ab.psiz() + PZ_VZ * A.psiz_plane + o;
-    pb[2] = ab.psiz() + PZ_VX * A.psiz_plane + o;
-  }
-  T rb[4] = {rtb[0], rtb[1], rtb[2], rtb[2]};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (pb[k]) {
-      const T P = *pb[k] + rb[k];
-      *pb[k] = cb[k] * P;
-      rb[k] = rb[k] * ik[k] + ca[k] * P;
-    }
-    rbar[k * np + c] = rb[k];
-  }
-}
-
-// C15 and C35 gather the half-node products of the four means they enter
-// (as k_gather does for C55)
-template <typename T>
-__global__ void k_tti_gather(const T *q15, const T *q35, double *g15, double *g35, int nx, int nz) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= nx || j >= nz) return;
-  const long long c = (long long)j * nx + i;
-  double t15 = 0, t35 = 0;
-  for (int dj = 0; dj <= 1; ++dj)
-    for (int di = 0; di <= 1; ++di) {
-      const int ii = i - di, jj = j - dj;
-      if (ii >= 0 && jj >= 0) {
-        t15 += q15[(long long)jj * nx + ii];
-        t35 += q35[(long long)jj * nx + ii];
+      for (int k = 0; k < V; ++k) {
+        bxz.v[k] = q0.w[k + 1];
+        eb[2].v[k] = T(0.25) * (c55.v[k] + right_of(c55, k, cc[V]) + c55d.v[k] + right_of(c55d, k, cc[G::WC + V])) *
+                     bxz.v[k];
       }
     }
-  g15[c] += 0.25 * t15;
-  g35[c] += 0.25 * t35;
-}
-
-// v += -D^T rbar over the update region (its taps reach at most L cells,
-// so they stay inside the planes; rbar is zero outside the region)
-template <typename T>
-__global__ void k_rates_t(AdjArgs<T> A, Slot<T> ab, const T *rbar) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + L;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + L;
-  if (i >= A.nx - L || j >= A.nz - L) return;
-  const int nx = A.nx;
-  const long long c = (long long)j * nx + i, np = A.np;
-  const T vx = ab.vx()[c], vz = ab.vz()[c];
-  ab.vx()[c] = vx - (tap_p(rbar, c, 1, A.Dx) + tap_m(rbar + 2 * np, c, nx, A.Dz));
-  ab.vz()[c] = vz - (tap_p(rbar + np, c, nx, A.Dz) + tap_m(rbar + 3 * np, c, 1, A.Dx));
-}
-
-// residual at the receivers of step it: vbar += d - obs
-template <typename T>
-__global__ void k_residual(Slot<T> ab, Slot<T> x1, const int2 *rec, int nrec, const T *obs, int ont,
-                           int it, int nx) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nrec) return;
-  const long long c = (long long)rec[r].y * nx + rec[r].x;
-  atomicAdd(ab.vx() + c, x1.vx()[c] - obs[(long long)r * ont + it]);
-  atomicAdd(ab.vz() + c, x1.vz()[c] - obs[(long long)(nrec + r) * ont + it]);
-}
-
-// V^T per cell: dbar (4 planes: sxx-x, sxz-z, sxz-x, szz-z) and the
-// buoyancy-gradient terms h (2 planes)
-template <typename T>
-__global__ void __launch_bounds__(256) k_vel_t(AdjArgs<T> A, Slot<T> x0, Slot<T> ab, T *dbar, T *h) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + L;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y + L;
-  if (i >= A.nx - L || j >= A.nz - L) return;
-  const int nx = A.nx, nz = A.nz;
-  const long long c = (long long)j * nx + i, np = A.np;
-  T d[4];
-  d[0] = tap_p(x0.sxx(), c, 1, A.Dx);   // ddxp sxx   (x, half)
-  d[1] = tap_m(x0.sxz(), c, nx, A.Dz);  // ddzm sxz   (z, integer)
-  d[2] = tap_m(x0.sxz(), c, 1, A.Dx);   // ddxm sxz   (x, integer)
-  d[3] = tap_p(x0.szz(), c, nx, A.Dz);  // ddzp szz   (z, half)
-  T ik[4] = {1, 1, 1, 1}, ca[4] = {0, 0, 0, 0}, cb[4] = {0, 0, 0, 0};
-  T *pb[4] = {nullptr, nullptr, nullptr, nullptr};
-  const int xs = strip_x(i, nx, A.Lx, A.Rx), zs = strip_z(j, nz, A.Tz, A.Bz);
-  T pn;
-  if (xs >= 0) {
-    const long long o = (long long)j * A.wx + xs;
-    ik[0] = A.tx[T_IKH * nx + i]; ca[0] = A.tx[T_AH * nx + i]; cb[0] = A.tx[T_BH * nx + i];
-    ik[2] = A.tx[T_IK * nx + i]; ca[2] = A.tx[T_A * nx + i]; cb[2] = A.tx[T_B * nx + i];
-    d[0] = cpml_fwd(d[0], x0.psix()[PX_SXX * A.psix_plane + o], ca[0], cb[0], ik[0], &pn);
-    d[2] = cpml_fwd(d[2], x0.psix()[PX_SXZ * A.psix_plane + o], ca[2], cb[2], ik[2], &pn);
-    pb[0] = ab.psix() + PX_SXX * A.psix_plane + o;
-    pb[2] = ab.psix() + PX_SXZ * A.psix_plane + o;
-  }
-  if (zs >= 0) {
-    const long long o = (long long)zs * nx + i;
-    ik[1] = A.tz[T_IK * nz + j]; ca[1] = A.tz[T_A * nz + j]; cb[1] = A.tz[T_B * nz + j];
-    ik[3] = A.tz[T_IKH * nz + j]; ca[3] = A.tz[T_AH * nz + j]; cb[3] = A.tz[T_BH * nz + j];
-    d[1] = cpml_fwd(d[1], x0.psiz()[PZ_SXZ * A.psiz_plane + o], ca[1], cb[1], ik[1], &pn);
-    d[3] = cpml_fwd(d[3], x0.psiz()[PZ_SZZ * A.psiz_plane + o], ca[3], cb[3], ik[3], &pn);
-    pb[1] = ab.psiz() + PZ_SXZ * A.psiz_plane + o;
-    pb[3] = ab.psiz() + PZ_SZZ * A.psiz_plane + o;
-  }
-  T pbo[4];
+    {
+      const T *a = box(SM::C15) + o;
+      const Row3<T> a0 = ldrow3(a), ap = ldrow3(a + W), am = ldrow3(a - W);
+      const Row3<T> sx0 = ldrow3(b0), sxp = ldrow3(b0 + W);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) pbo[k] = pb[k] ? *pb[k] : T(0);
-  const T bx = T(2) / (A.rho[c] + A.rho[c + 1]);
-  const T bz = T(2) / (A.rho[c] + A.rho[c + nx]);
-  const T vbx = ab.vx()[c], vbz = ab.vz()[c];
-  // d(vx')/d rho = dt * (-bx^2 / 2) * div
-  h[c] = A.dt * T(-0.5) * bx * bx * (d[0] + d[1]) * vbx;
-  h[np + c] = A.dt * T(-0.5) * bz * bz * (d[2] + d[3]) * vbz;
-  T db[4] = {A.dt * bx * vbx, A.dt * bx * vbx, A.dt * bz * vbz, A.dt * bz * vbz};
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (pb[k]) {
-      const T P = pbo[k] + db[k];
-      *pb[k] = cb[k] * P;
-      db[k] = db[k] * ik[k] + ca[k] * P;
+      for (int k = 0; k < V; ++k) {
+        const T sx = mean_of(a0, ap, k + 1) * q0.w[k + 1] + mean_of(a0, ap, k) * q0.w[k] +
+                     mean_of(am, a0, k + 1) * qm.w[k + 1] + mean_of(am, a0, k) * qm.w[k];
+        eb[0].v[k] += T(0.25) * sx;
+        eb[2].v[k] += T(0.25) * (a0.w[k + 1] * sx0.w[k + 1] + a0.w[k + 2] * sx0.w[k + 2] +
+                                 ap.w[k + 1] * sxp.w[k + 1] + ap.w[k + 2] * sxp.w[k + 2]);
+      }
     }
-    dbar[k * np + c] = db[k];
+    {
+      const T *a = box(SM::C35) + o;
+      const Row3<T> a0 = ldrow3(a), ap = ldrow3(a + W), am = ldrow3(a - W);
+      const Row3<T> sz0 = ldrow3(b0 + RP), szp = ldrow3(b0 + RP + W);
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const T sz = mean_of(a0, ap, k + 1) * q0.w[k + 1] + mean_of(a0, ap, k) * q0.w[k] +
+                     mean_of(am, a0, k + 1) * qm.w[k + 1] + mean_of(am, a0, k) * qm.w[k];
+        eb[1].v[k] += T(0.25) * sz;
+        eb[2].v[k] += T(0.25) * (a0.w[k + 1] * sz0.w[k + 1] + a0.w[k + 2] * sz0.w[k + 2] +
+                                 ap.w[k + 1] * szp.w[k + 1] + ap.w[k + 2] * szp.w[k + 2]);
+        c35own.v[k] = a0.w[k + 1];
+      }
+    }
   }
-}
-
-// force sources: their buoyancy factor also depends on rho
-template <typename T>
-__global__ void k_force_rho_t(AdjArgs<T> A, Slot<T> ab, const int4 *src, const T *amp, int nsrc,
-                              const T *wav, int wnt, int it, T *h) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nsrc) return;
-  const int4 s = src[q];
-  if (s.z == VI_SRC_EXPLOSIVE) return;
-  const long long c = (long long)s.y * A.nx + s.x;
-  const T f = it < wnt ? amp[q] * wav[(long long)q * wnt + it] : T(0);
-  if (s.z == VI_SRC_FORCE_X) {
-    const T bx = T(2) / (A.rho[c] + A.rho[c + 1]);
-    atomicAdd(h + c, A.dt * T(-0.5) * bx * bx * f * ab.vx()[c]);
+  {  // forward rates at the cell and the means its update used
+    const Row3<T> z0 = ldrow3(f0 + 2 * RP), zm = ldrow3(f0 + 2 * RP - W);
+    T ebx1[V + 1];
+#pragma unroll
+    for (int k = 0; k <= V; ++k) ebx1[k] = mean_of(zm, z0, k);
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      ebxz.v[k] = ebx1[k];
+      exz.v[k] = z0.w[k + 1];
+    }
+    const Row3<T> x0 = ldrow3(f0), xp = ldrow3(f0 + W);
+    Row3<T> w0 = ldrow3(f0 + RP);
+    const Row3<T> wp = ldrow3(f0 + RP + W);
+    if (surf) {  // the surface relation: ezz of the group and of the cell after it
+      const T *a = box(SM::C35) + o;
+#pragma unroll
+      for (int k = 0; k <= V; ++k)
+        if (t.gi0 + k < A.nx - L)
+          w0.w[k + 1] = -(ldn1(A.c13 + c + k) * x0.w[k + 1] + a[k] * ebx1[k]) / ldn1(A.c33 + c + k);
+    }
+    // accumulators: plane 0 TAU, 1 Q55, 2 C11, 3 C13, 4 C33, 5 C15, 6 C35, 7 Q15, 8 Q35
+    acc_add<T>(ai + PL, ao + np, [&](int k, double g) { return fma((double)bxz.v[k], (double)exz.v[k], g); });
+    acc_add<T>(ai + 7 * PL, ao + 7 * np,
+               [&](int k, double g) { return fma((double)bxz.v[k], (double)mean_of(x0, xp, k + 1), g); });
+    acc_add<T>(ai + 8 * PL, ao + 8 * np,
+               [&](int k, double g) { return fma((double)bxz.v[k], (double)mean_of(w0, wp, k + 1), g); });
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      exx.v[k] = x0.w[k + 1];
+      ezz.v[k] = w0.w[k + 1];
+    }
+  }
+  acc_add<T>(ai + 2 * PL, ao + 2 * np, [&](int k, double g) { return fma((double)bxx.v[k], (double)exx.v[k], g); });
+  acc_add<T>(ai + 5 * PL, ao + 5 * np, [&](int k, double g) { return fma((double)bxx.v[k], (double)ebxz.v[k], g); });
+  if (!surf) {
+    acc_add<T>(ai + 3 * PL, ao + 3 * np, [&](int k, double g) {
+      return fma((double)bxx.v[k], (double)ezz.v[k], fma((double)bzz.v[k], (double)exx.v[k], g));
+    });
+    acc_add<T>(ai + 4 * PL, ao + 4 * np, [&](int k, double g) { return fma((double)bzz.v[k], (double)ezz.v[k], g); });
+    acc_add<T>(ai + 6 * PL, ao + 6 * np, [&](int k, double g) { return fma((double)bzz.v[k], (double)ebxz.v[k], g); });
   } else {
-    const T bz = T(2) / (A.rho[c] + A.rho[c + A.nx]);
-    atomicAdd(h + A.np + c, A.dt * T(-0.5) * bz * bz * f * ab.vz()[c]);
+    // the adjoint of the surface ezz moves to exx of the cell and to exz of
+    // the cell and its left neighbour, with its stiffness terms (bzz = 0)
+    Pk<T> zb = eb[1], wz;  // wz: C35 / C33 zb
+    if (t.gi0 + V > A.nx - L) zero_outside(zb, A.nx - L - t.gi0);
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      wz.v[k] = c35own.v[k] / C33.v[k] * zb.v[k];
+      eb[0].v[k] -= C13.v[k] / C33.v[k] * zb.v[k];
+    }
+#pragma unroll
+    for (int k = 0; k < V; ++k) eb[2].v[k] -= T(0.25) * (wz.v[k] + right_of(wz, k, wr * zr));
+    eb[1] = splat<T>(T(0));
+    acc_add<T>(ai + 3 * PL, ao + 3 * np, [&](int k, double g) {
+      return fma((double)bxx.v[k], (double)ezz.v[k], g) - (double)zb.v[k] * (double)exx.v[k] / (double)C33.v[k];
+    });
+    acc_add<T>(ai + 4 * PL, ao + 4 * np,
+               [&](int k, double g) { return g - (double)zb.v[k] * (double)ezz.v[k] / (double)C33.v[k]; });
+    acc_add<T>(ai + 6 * PL, ao + 6 * np,
+               [&](int k, double g) { return g - (double)zb.v[k] * (double)ebxz.v[k] / (double)C33.v[k]; });
   }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    eb[k] = pscale(A.dt, eb[k]);
+    if (t.gi0 + V > A.nx - L) zero_outside(eb[k], A.nx - L - t.gi0);
+  }
+  if (N > 0)
+    acc_add<T>(ai, ao, [&](int k, double g) {
+      const double u = fma((double)eb[1].v[k], (double)rs[1].v[k], (double)eb[0].v[k] * (double)rs[0].v[k]);
+      return g + fma((double)eb[2].v[k], (double)rs[2].v[k], u);
+    });
+  adj_memory<T, N>(A, [&](int q) { return mb[q]; }, mbar + c, pxb, pzb, strips_of(A, t.gi0, t.j), t, c, surf, tau, eb,
+                   rbar);
 }
 
-// grho gathers h of the two velocity nodes each density value feeds;
-// gc55 gathers the 4 half-node terms q that average mu around each cell
-template <typename T>
-__global__ void k_gather(const T *h, double *grho, const T *q, double *gc55, int nx, int nz) {
-  pdl_wait();  // launched while the previous kernel drains
+// The gradient planes from the accumulators: dt applied, the buoyancy terms
+// spread over the two densities of each velocity node and the half-node terms
+// over the four cells of each mean.  ISO: C11 = C33 = lambda + 2 mu, C13 =
+// lambda, C55 = mu.
+__global__ void k_adj_finish(int kind, int nx, int nz, int ld, double dt, const double *acc, int accumulate,
+                             double *grad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= nx || j >= nz) return;
-  const long long c = (long long)j * nx + i, np = (long long)nx * nz;
-  const double gr = grho[c], g55 = gc55[c];
-  double s = (double)h[c] + (double)h[np + c];
-  if (i > 0) s += h[c - 1];
-  if (j > 0) s += h[np + c - nx];
-  double t = 0;
-  for (int dj = 0; dj <= 1; ++dj)
-    for (int di = 0; di <= 1; ++di) {
-      const int ii = i - di, jj = j - dj;
-      if (ii >= 0 && jj >= 0) t += q[(long long)jj * nx + ii];
-    }
-  grho[c] = gr + s;
-  gc55[c] = g55 + 0.25 * t;
-}
-
-// sigma += -D^T dbar over every cell the velocity stencil reads (ghost rows
-// included; the images^T of the previous step folds them)
-template <typename T>
-__global__ void k_div_t(AdjArgs<T> A, Slot<T> ab, const T *dbar) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= A.nx || j >= A.nz) return;
-  const int nx = A.nx, nz = A.nz;
-  const long long c = (long long)j * nx + i, np = A.np;
-  const T sxx = ab.sxx()[c], sxz = ab.sxz()[c], szz = ab.szz()[c];
-  if (i >= L && i < nx - L && j >= L && j < nz - L) {  // taps inside the planes: unchecked
-    ab.sxx()[c] = sxx - tap_m(dbar, c, 1, A.Dx);
-    ab.sxz()[c] = sxz - (tap_p(dbar + np, c, nx, A.Dz) + tap_p(dbar + 2 * np, c, 1, A.Dx));
-    ab.szz()[c] = szz - tap_m(dbar + 3 * np, c, nx, A.Dz);
+  const long long np = (long long)ld * nz, c = (long long)j * ld + i, npo = (long long)nx * nz;
+  auto half = [&](int q) {  // 1/4 of the four cells whose mean reads this one
+    const double *p = acc + q * np + c;
+    double t = p[0];
+    if (i > 0) t += p[-1];
+    if (j > 0) t += p[-ld];
+    if (i > 0 && j > 0) t += p[-ld - 1];
+    return 0.25 * dt * t;
+  };
+  double g[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  const double *h = acc + ACC_HX * np + c, *v = acc + ACC_HZ * np + c;
+  g[0] = h[0] + v[0] + (i > 0 ? h[-1] : 0.0) + (j > 0 ? v[-ld] : 0.0);
+  g[7] = acc[ACC_TAU * np + c];
+  const double g11 = dt * acc[ACC_11 * np + c], g13 = dt * acc[ACC_13 * np + c];
+  if (kind == VI_MEDIUM_ISO) {
+    g[2] = g11 + g13;
+    g[6] = 2.0 * g11 + half(ACC_Q55);
   } else {
-    ab.sxx()[c] = sxx - tap_m_b(dbar, i, j, nx, nz, 0, A.Dx);
-    ab.sxz()[c] = sxz - (tap_p_b(dbar + np, i, j, nx, nz, 1, A.Dz) + tap_p_b(dbar + 2 * np, i, j, nx, nz, 0, A.Dx));
-    ab.szz()[c] = szz - tap_m_b(dbar + 3 * np, i, j, nx, nz, 1, A.Dz);
+    g[1] = g11;
+    g[2] = g13;
+    g[4] = dt * acc[ACC_33 * np + c];
+    g[6] = half(ACC_Q55);
   }
-}
-
-// ---- 4-cell forms of the transposed derivatives (nx % 4 == 0, 16-byte
-// aligned planes): one thread per group of 4 x-adjacent cells, x taps from
-// a 12-value row window of three 128-bit loads, z taps as one 128-bit load
-// per row; per cell the same arithmetic as the scalar kernels.
-template <typename T>
-__device__ __forceinline__ void win12(const T *p, T (&o)[12]) {  // p[-4 .. +7]
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const Q4<T> v = ldc4(p - 4 + 4 * q);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) o[4 * q + k] = v.v[k];
+  if (kind == VI_MEDIUM_TTI) {
+    g[3] = dt * acc[ACC_15 * np + c] + half(ACC_Q15);
+    g[5] = dt * acc[ACC_35 * np + c] + half(ACC_Q35);
   }
-}
-template <typename T>
-__device__ __forceinline__ Q4<T> zp4(const T *p, long long s, const T *D) {  // ddzp form
-  Q4<T> acc = mul4(splat4<T>(D[0]), sub4(ldc4(p + s), ldc4(p)));
+  double *o = grad + (long long)j * nx + i;
 #pragma unroll
-  for (int q = 1; q < 4; ++q) acc = fma4(splat4<T>(D[q]), sub4(ldc4(p + (q + 1) * s), ldc4(p - q * s)), acc);
-  return acc;
-}
-template <typename T>
-__device__ __forceinline__ Q4<T> zm4(const T *p, long long s, const T *D) {  // ddzm form
-  Q4<T> acc = mul4(splat4<T>(D[0]), sub4(ldc4(p), ldc4(p - s)));
-#pragma unroll
-  for (int q = 1; q < 4; ++q) acc = fma4(splat4<T>(D[q]), sub4(ldc4(p + q * s), ldc4(p - (q + 1) * s)), acc);
-  return acc;
+  for (int q = 0; q < 8; ++q) o[q * npo] = accumulate ? o[q * npo] + g[q] : g[q];
 }
 
-// v += -D^T rbar, 4 cells per thread over the update region
+// FP64 misfit: 1/2 sum (d - obs)^2, one partial sum per block, added in block
+// order by the last kernel's thread (a fixed order).  One block alone took 53
+// us for 82 k samples.
+constexpr int kMisfitBlocks = 64;
 template <typename T>
-__global__ void __launch_bounds__(256) k_rates_t4(AdjArgs<T> A, Slot<T> ab, const T *rbar) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int gi0 = L + 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = L + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  if (gi0 >= A.nx - L || j >= A.nz - L) return;
-  const int nx = A.nx;
-  const long long g = (long long)j * nx + gi0, np = A.np;
-  T w0[12], w3[12];
-  win12(rbar + g, w0);
-  win12(rbar + 3 * np + g, w3);
-  const Q4<T> x0 = dps4(w0, A.Dx), x3 = dms4(w3, A.Dx);
-  const Q4<T> z2 = zm4(rbar + 2 * np + g, nx, A.Dz), z1 = zp4(rbar + np + g, nx, A.Dz);
-  const Q4<T> vx = ldc4(ab.vx() + g), vz = ldc4(ab.vz() + g);
-  stg4(ab.vx() + g, sub4(vx, add4(x0, z2)));
-  stg4(ab.vz() + g, sub4(vz, add4(z1, x3)));
-}
-
-// sigma += -D^T dbar, 4 cells per thread over every cell (groups whose taps
-// leave the planes take the checked scalar form)
-template <typename T>
-__global__ void __launch_bounds__(256) k_div_t4(AdjArgs<T> A, Slot<T> ab, const T *dbar) {
-  pdl_wait();  // launched while the previous kernel drains
-  const int gi0 = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int nx = A.nx, nz = A.nz;
-  if (gi0 >= nx || j >= nz) return;
-  const long long g = (long long)j * nx + gi0, np = A.np;
-  if (gi0 >= L && gi0 + 3 < nx - L && j >= L && j < nz - L) {
-    T w0[12], w2[12];
-    win12(dbar + g, w0);
-    win12(dbar + 2 * np + g, w2);
-    const Q4<T> sxx = ldc4(ab.sxx() + g), sxz = ldc4(ab.sxz() + g), szz = ldc4(ab.szz() + g);
-    stg4(ab.sxx() + g, sub4(sxx, dms4(w0, A.Dx)));
-    stg4(ab.sxz() + g, sub4(sxz, add4(zp4(dbar + np + g, nx, A.Dz), dps4(w2, A.Dx))));
-    stg4(ab.szz() + g, sub4(szz, zm4(dbar + 3 * np + g, nx, A.Dz)));
-  } else {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int i = gi0 + k;
-      const long long c = g + k;
-      const T sxx = ab.sxx()[c], sxz = ab.sxz()[c], szz = ab.szz()[c];
-      ab.sxx()[c] = sxx - tap_m_b(dbar, i, j, nx, nz, 0, A.Dx);
-      ab.sxz()[c] = sxz - (tap_p_b(dbar + np, i, j, nx, nz, 1, A.Dz) + tap_p_b(dbar + 2 * np, i, j, nx, nz, 0, A.Dx));
-      ab.szz()[c] = szz - tap_m_b(dbar + 3 * np, i, j, nx, nz, 1, A.Dz);
-    }
-  }
-}
-
-// FP64 misfit: 1/2 sum (d - obs)^2 (one block, deterministic order)
-template <typename T>
-__global__ void k_misfit(const T *tr, const T *obs, long long n, double *out) {
+__global__ void k_misfit(const T *tr, const T *obs, long long n, double *part) {
   __shared__ double red[256];
   double s = 0;
-  for (long long k = threadIdx.x; k < n; k += blockDim.x) {
+  for (long long k = blockIdx.x * 256LL + threadIdx.x; k < n; k += kMisfitBlocks * 256LL) {
     const double d = (double)tr[k] - (double)obs[k];
     s += d * d;
   }
@@ -804,10 +1209,15 @@ __global__ void k_misfit(const T *tr, const T *obs, long long n, double *out) {
     if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *out = 0.5 * red[0];
+  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+}
+__global__ void k_misfit_sum(const double *part, double *out) {
+  double s = 0;
+  for (int k = 0; k < kMisfitBlocks; ++k) s += part[k];
+  *out = 0.5 * s;
 }
 
-// ISO fold and the (vp, vs, rho, 1/Q) chain rule
+// The (vp, vs, rho, 1/Q) chain rule
 __global__ void k_velocity_grad(int kind, long long np, const double *g, const double *vp,
                                 const double *vs, const double *rho, const double *eps,
                                 const double *delta, double tau_scale, double *out) {
@@ -914,17 +1324,6 @@ __global__ void k_tti_param_grad(long long np, const double *g, const double *vp
   out[3 * np + c] = g[7 * np + c] * tau_scale;  // dJ/d(1/Q)
 }
 
-__global__ void k_fold_iso(long long np, double *g) {
-  const long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (c >= np) return;
-  // C11 = C33 = lambda + 2 mu, C13 = lambda, C55 = mu
-  const double g11 = g[1 * np + c], g13 = g[2 * np + c], g33 = g[4 * np + c], g55 = g[6 * np + c];
-  g[2 * np + c] = g11 + g13 + g33;
-  g[6 * np + c] = 2 * (g11 + g33) + g55;
-  g[1 * np + c] = 0;
-  g[4 * np + c] = 0;
-}
-
 }  // namespace
 
 template <typename T>
@@ -940,109 +1339,121 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
   if (!grad) return set_error(VI_ERR_ARG, "gradient: grad buffer is NULL");
   if (nt <= 0) return set_error(VI_ERR_ARG, "gradient: nt must be positive");
   if ((rc = cuda_check(cudaSetDevice(p->device), "cudaSetDevice"))) return rc;
-  const long long np = (long long)c.nx * c.nz;
-  const int N = c.nsls;
-  const long long slot = Slot<T>::size(np, p->psix_plane, p->psiz_plane, N);
+  const int N = c.nsls, ld = (c.nx + 3) / 4 * 4;
+  // every plane of the workspace has rows of ld cells, so odd grids take the
+  // same vector kernels
+  const long long np = (long long)ld * c.nz;
+  const long long px = (long long)p->wx * c.nz, pz = (long long)ld * p->hz;
+  const long long slot = Slot<T>::size(np, px, pz, N);
   const int nrec = shot->nrec;
   const long long ntr = 2LL * nrec * nt;
-  const long long scratch = 4 * np + np + 2 * np + 6 * np + (tti ? 5 * np : 0);
+  // the medium where its planes are not laid out so already
+  const void *med[8] = {m->rho, m->c11, m->c13, m->c15, m->c33, m->c35, m->c55, m->tau};
+  bool copy_med = ld != c.nx;
+  int nmed = 0;
+  for (const void *q : med) {
+    copy_med |= ((uintptr_t)q & 15) != 0;
+    nmed += q != nullptr;
+  }
+  const long long wide = sizeof(double) / sizeof(T);
+  const long long scratch = (8 + (tti ? 6 : 0) + acc_planes(c.medium) * wide + (copy_med ? nmed : 0)) * np;
   // K = 0: every state of the forward sweep kept in HBM when the sweep fits
   // in 60 % of the device's memory and in what is free (1024 x 512 x 3000
   // VTI FP32: 88 GB), so the adjoint reads each step's states and nothing
   // is recomputed; else checkpoints every ceil(sqrt(nt)) steps
   bool keep_all = false;
   if (K <= 0) {
-    size_t fr = 0, tot = 0;
-    if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) {
-      const size_t all = sizeof(T) * ((size_t)(nt + 2) * slot + scratch + ntr) + 64;
-      const size_t avail = fr + p->fwd_bytes;
-      keep_all = all <= (size_t)(0.6 * (double)tot) && all + (2ull << 30) <= avail;
+    const size_t all = sizeof(T) * ((size_t)(nt + 2) * slot + scratch + ntr) + 64;
+    if (p->device_bytes > 0 && all <= p->fwd_bytes) {
+      // the workspace holds the sweep already: nothing to ask the driver
+      // (cudaMemGetInfo took up to 10 ms of a 10 ms gradient)
+      keep_all = all <= (size_t)(0.6 * (double)p->device_bytes);
+    } else {
+      size_t fr = 0, tot = 0;
+      if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) {
+        const size_t avail = fr + p->fwd_bytes;
+        keep_all = all <= (size_t)(0.6 * (double)tot) && all + (2ull << 30) <= avail;
+        p->device_bytes = tot;
+      }
+      cudaGetLastError();
     }
-    cudaGetLastError();
     K = (int)std::ceil(std::sqrt((double)nt));
   }
   if (K > nt) K = nt;
   const int nck = keep_all ? nt + 1 : (nt + K - 1) / K;
   // workspace: checkpoints (keep_all: every state) | segment (K + 1 slots; none when keep_all) |
-  // adjoint slot | scratch (4 rbar/dbar, q, 2 h, 6 plain (TTI: also the forward effective rates of
-  // the adjoint sweep), TTI: 3 effective-rate adjoints, q15, q35) | traces
-  const size_t need = sizeof(T) * ((size_t)(nck + (keep_all ? 0 : K + 1) + 1) * slot + scratch + ntr) + 64;
+  // adjoint slot | rbar, dbar (4 planes each) | TTI: forward effective rates (6 planes) | FP64
+  // accumulators | medium copies | traces | misfit
+  const size_t need = sizeof(T) * ((size_t)(nck + (keep_all ? 0 : K + 1) + 1) * slot + scratch + ntr) + 64 + 8 * kMisfitBlocks;
   size_t have = p->fwd_bytes;
   if ((rc = ensure_buffer(p, &p->fwd, &have, need))) return rc;
   p->fwd_bytes = have;
   T *ck = (T *)p->fwd;
   T *seg = keep_all ? ck : ck + (size_t)nck * slot;
   T *adj = keep_all ? ck + (size_t)nck * slot : seg + (size_t)(K + 1) * slot;
-  T *rbar = adj + slot;   // also dbar
-  T *q = rbar + 4 * np;
-  T *h = q + np;
-  T *pscr = h + 2 * np;   // plain-path scratch (6 planes)
-  T *teb = pscr + 6 * np;  // TTI: effective-rate adjoints (3 planes), q15, q35
-  T *tq15 = teb + 3 * np, *tq35 = tq15 + np;
-  T *tr = pscr + 6 * np + (tti ? 5 * np : 0);
-  auto mk = [&](T *b) { return Slot<T>{b, np, p->psix_plane, p->psiz_plane, N}; };
+  T *rbar = adj + slot, *dbar = rbar + 4 * np, *fe = dbar + 4 * np;
+  double *acc = (double *)(fe + (tti ? 6 * np : 0));
+  T *pmed = (T *)(acc + acc_planes(c.medium) * np);
+  T *tr = pmed + (copy_med ? nmed * np : 0);
+  auto mk = [&](T *b) { return Slot<T>{b, np, px, pz, N}; };
   if ((rc = stage_shot<T>(p, shot, st))) return rc;
-  // plain forward step on a slot, in place (bind() points it at the slot)
+  vi_medium mw = *m;
+  if (copy_med) {
+    const void **slotp[8] = {&mw.rho, &mw.c11, &mw.c13, &mw.c15, &mw.c33, &mw.c35, &mw.c55, &mw.tau};
+    const T *src[8];
+    T *dst[8];
+    int q = 0;
+    for (int k = 0; k < 8; ++k)
+      if (med[k]) {
+        src[q] = (const T *)med[k];
+        dst[q] = pmed + q * np;
+        *slotp[k] = dst[q];
+        ++q;
+      }
+    if ((rc = cuda_check(cudaMemsetAsync(pmed, 0, nmed * np * sizeof(T), st), "zero medium copies"))) return rc;
+    if ((rc = copy_planes<T>(src, dst, nmed, c.nx, ld, c.nx, c.nz, st))) return rc;
+  }
+  // a forward step on slots (bind() points it at them)
   vi_fields fdummy{};
   fdummy.vx = fdummy.vz = fdummy.sxx = fdummy.szz = fdummy.sxz = (void *)ck;
   fdummy.m = ck;
   fdummy.m_plane_stride = np;
-  StepArgs<T> a = make_args<T>(p, m, &fdummy);
-  PlainExtras<T> x;
-  x.scratch = pscr;
-  x.fs = c.free_surface;
-  x.src = (const int4 *)p->dsrc;
-  x.amp = (const T *)p->damp;
-  x.nsrc = shot->nsrc;
-  x.wavelet = shot->nsrc ? (const T *)shot->wavelet_dev : nullptr;
-  x.wnt = shot->nsrc ? shot->wavelet_nt : 0;
-  x.rec = (const int2 *)p->drec;
-  x.nrec = nrec;
-  x.traces = nullptr;
-  x.tnt = nt;
-  auto bind = [&](StepArgs<T> &s, const Slot<T> &sl) {
-    s.vx = sl.vx(); s.vz = sl.vz(); s.sxx = sl.sxx(); s.szz = sl.szz(); s.sxz = sl.sxz();
-    s.m = sl.m(); s.mstride = np;
-    s.psix = s.psix_o = p->wx ? sl.psix() : nullptr;
-    s.psiz = s.psiz_o = p->hz ? sl.psiz() : nullptr;
-  };
+  StepArgs<T> a = make_args<T>(p, &mw, &fdummy);
+  a.ld = a.ldz = ld;
+  a.psix_plane = px;
+  a.psiz_plane = pz;
   const size_t sbytes = (size_t)slot * sizeof(T);
-  // plain-path scratch: cells outside the update region are read, never written
-  if ((rc = cuda_check(cudaMemsetAsync(pscr, 0, 6 * np * sizeof(T), st), "zero scratch"))) return rc;
-  // The two forward sweeps (traces + checkpoints, then the segment
-  // recompute) run on the split pair when the grid allows it (the same
-  // discrete step as the plain path the adjoint transposes, faster), else
-  // on the plain path.
+  // The forward sweeps (traces + checkpoints, then the segment recompute)
+  // run on the split pair, the same discrete step as the plain path the
+  // adjoint transposes.  TTI sweeps step out of place only (the TTI stress
+  // pass reads M and psi on a ring of neighbouring cells).
   using SG = SplitGeom<T>;
-  StepArgs<T> probe = a;
-  bind(probe, mk(seg));
-  // TTI sweeps step out of place only (the TTI stress pass reads M and psi
-  // on a ring of neighbouring cells, so it writes them to the other slot);
-  // the 4-cell transposed derivatives only need aligned planes
-  const bool split_ok = split_eligible<T>(p, probe);
-  const bool use_split = split_ok;
   using STG = SplitTtiGeom<T>;
   using SS = SplitStressGeom<T>;
-  FusedExtras<T> fx{}, fxs{};
+  using AG = AdjGeom<T>;
+  FusedExtras<T> fx{}, fxs{}, fxa{};
   SplitMaps ms{};
-  int ntiles = 0, sntiles = 0;
-  if (use_split) {
-    // velocity tiling and stress tiling, one buffer of lists
-    int ntx = 0, ntz = 0, sntx = 0, sntz = 0;
-    std::vector<int> off, soff;
-    std::vector<int4> ent, sent;
+  int ntiles = 0, sntiles = 0, antiles = 0;
+  {
+    // velocity, stress and adjoint tilings, one buffer of lists
+    int ntx = 0, ntz = 0, sntx = 0, sntz = 0, antx = 0, antz = 0;
+    std::vector<int> off, soff, aoff;
+    std::vector<int4> ent, sent, aent;
     build_tile_lists(c.nx, c.nz, SG::TX, SG::TZ, 0, shot, off, ent, ntx, ntz);
     build_tile_lists(c.nx, c.nz, tti ? STG::TX : SS::TX, tti ? STG::TZ : SS::TZ, 0, shot, soff, sent, sntx, sntz);
+    build_tile_lists(c.nx, c.nz, AG::TX, AG::TZ, 0, shot, aoff, aent, antx, antz);
     const int nvoff = (int)off.size();
     for (int v : soff) off.push_back(v + (int)ent.size());
     ent.insert(ent.end(), sent.begin(), sent.end());
+    const int naoff = (int)off.size();
+    for (int v : aoff) off.push_back(v + (int)ent.size());
+    ent.insert(ent.end(), aent.begin(), aent.end());
     int *d_off = nullptr;
     int4 *d_ent = nullptr;
     if ((rc = stage_tile_lists(p, off, ent, st, &d_off, &d_ent))) return rc;
+    antiles = antx * antz;
     ntiles = ntx * ntz;
     sntiles = sntx * sntz;
-    fxs.ntx = sntx;
-    fxs.tile_off = d_off + nvoff;
     fx.ntx = ntx;
     fx.fs = c.free_surface;
     fx.tile_off = d_off;
@@ -1054,50 +1465,27 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
     fx.tnt = nt;
     fx.err = (int *)p->errflag;
     fx.l2hint = l2_hints_fit(5LL * c.nx * c.nz * (long long)sizeof(T), p->l2_bytes);
-    const int sntx_keep = fxs.ntx;
-    const int *soff_keep = fxs.tile_off;
     fxs = fx;
-    fxs.ntx = sntx_keep;
-    fxs.tile_off = soff_keep;
+    fxs.ntx = sntx;
+    fxs.tile_off = d_off + nvoff;
+    fxa = fx;
+    fxa.ntx = antx;
+    fxa.tile_off = d_off + naoff;
   }
-  // One forward step of slot sl, in place, or (split pair, out != nullptr)
-  // from slot sl into slot *out, which then holds the next state.
+  // One forward step of slot sl, in place (ISO/VTI) or (out != nullptr) from
+  // slot sl into slot *out, which then holds the next state.
   auto fwd_step = [&](const Slot<T> &sl, int it, T *traces, bool pdl, const Slot<T> *out = nullptr) -> int {
-    if (!use_split) {
-      bind(a, sl);
-      x.traces = traces;
-      plain_step<T>(a, x, c.medium, it, st);
-      return VI_OK;
-    }
     StepArgs<T> b = a;
-    if (tti) {
-      // v and sigma copied into the output slot and stepped there in place;
-      // M and psi from the input slot to the output one
-      if (!out) return set_error(VI_ERR_ARG, "gradient: the TTI split step runs out of place");
-      int r2 = cuda_check(cudaMemcpyAsync(out->vx(), sl.vx(), 5 * (size_t)np * sizeof(T), cudaMemcpyDeviceToDevice, st),
-                          "state copy");
-      bind(b, *out);
-      b.m = sl.m();
-      b.mstride = np;
-      b.m_o = out->m();
-      b.mstride_o = np;
-      b.psix = p->wx ? sl.psix() : nullptr;
-      b.psiz = p->hz ? sl.psiz() : nullptr;
-      b.psix_o = p->wx ? out->psix() : nullptr;
-      b.psiz_o = p->hz ? out->psiz() : nullptr;
-      fx.it = fxs.it = it;
-      fx.traces = fxs.traces = traces;
-      if (!r2) r2 = encode_map(&ms.a, out->vx(), (int)sizeof(T), c.nx, c.nz, 1, 0, STG::BW, STG::BH, 1);
-      if (!r2) r2 = encode_map(&ms.b, out->vz(), (int)sizeof(T), c.nx, c.nz, 1, 0, STG::BW, STG::BH, 1);
-      if (!r2) r2 = launch_split_vel<T>(b, fx, ntiles, st, false);
-      if (!r2) r2 = launch_split_stress_tti<T>(b, fxs, ms, sntiles, st, true);
-      return r2;
-    }
-    bind(b, sl);
+    b.vx = sl.vx(); b.vz = sl.vz(); b.sxx = sl.sxx(); b.szz = sl.szz(); b.sxz = sl.sxz();
+    b.m = sl.m();
+    b.mstride = np;
+    b.psix = b.psix_o = p->wx ? sl.psix() : nullptr;
+    b.psiz = b.psiz_o = p->hz ? sl.psiz() : nullptr;
     if (out) {
       b.vx_o = out->vx(); b.vz_o = out->vz();
       b.sxx_o = out->sxx(); b.szz_o = out->szz(); b.sxz_o = out->sxz();
-      b.m_o = out->m(); b.mstride_o = np;
+      b.m_o = out->m();
+      b.mstride_o = np;
       b.psix_o = p->wx ? out->psix() : nullptr;
       b.psiz_o = p->hz ? out->psiz() : nullptr;
     }
@@ -1105,10 +1493,13 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
     fx.traces = fxs.traces = traces;
     // the stress pass stages the new velocities: those of the output state
     T *nvx = out ? out->vx() : b.vx, *nvz = out ? out->vz() : b.vz;
-    int r2 = encode_map(&ms.a, nvx, (int)sizeof(T), c.nx, c.nz, 1, 0, SS::BW, SS::BH, 1);
-    if (!r2) r2 = encode_map(&ms.b, nvz, (int)sizeof(T), c.nx, c.nz, 1, 0, SS::BW, SS::BH, 1);
+    const int bw = tti ? STG::BW : SS::BW, bh = tti ? STG::BH : SS::BH;
+    int r2 = encode_map(&ms.a, nvx, (int)sizeof(T), ld, c.nz, 1, 0, bw, bh, 1);
+    if (!r2) r2 = encode_map(&ms.b, nvz, (int)sizeof(T), ld, c.nz, 1, 0, bw, bh, 1);
     if (!r2) r2 = launch_split_vel<T>(b, fx, ntiles, st, pdl);
-    if (!r2) r2 = launch_split_stress<T>(c.medium, b, fxs, ms, sntiles, st, true);
+    if (!r2)
+      r2 = tti ? launch_split_stress_tti<T>(b, fxs, ms, sntiles, st, true)
+               : launch_split_stress<T>(c.medium, b, fxs, ms, sntiles, st, true);
     return r2;
   };
   // the caller's hook after every enqueued step (a server's slicing)
@@ -1136,16 +1527,8 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
   if (keep_all) {
     NvtxRange nr("vi_gradient: forward sweep, every state kept");
     for (int it = 0; it < nt; ++it) {
-      T *nxt = ck + (size_t)(it + 1) * slot;
-      if (use_split) {
-        const Slot<T> out = mk(nxt);
-        if ((rc = fwd_step(mk(ck + (size_t)it * slot), it, tr, it > 0, &out))) return rc;
-      } else {
-        if ((rc = cuda_check(cudaMemcpyAsync(nxt, ck + (size_t)it * slot, sbytes, cudaMemcpyDeviceToDevice, st),
-                             "state copy")))
-          return rc;
-        if ((rc = fwd_step(mk(nxt), it, tr, false))) return rc;
-      }
+      const Slot<T> out = mk(ck + (size_t)(it + 1) * slot);
+      if ((rc = fwd_step(mk(ck + (size_t)it * slot), it, tr, it > 0, &out))) return rc;
       if ((rc = yield(1))) return rc;
     }
   } else {
@@ -1156,9 +1539,9 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
                                              cudaMemcpyDeviceToDevice, st),
                              "checkpoint")))
           return rc;
-      if (tti && use_split) {  // out of place: between the segment's first two slots
+      if (tti) {  // out of place: between the segment's first two slots
         const Slot<T> nxt = mk(cur.base == seg ? seg + slot : seg);
-        if ((rc = fwd_step(cur, it, tr, false, &nxt))) return rc;
+        if ((rc = fwd_step(cur, it, tr, it % K != 0, &nxt))) return rc;
         cur = nxt;
       } else if ((rc = fwd_step(cur, it, tr, it % K != 0))) {
         return rc;
@@ -1173,11 +1556,12 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
   }
   double *dmis = (double *)(tr + ntr);
   dmis = (double *)(((uintptr_t)dmis + 15) / 16 * 16);
-  k_misfit<T><<<1, 256, 0, st>>>(tr, obs, ntr, dmis);
+  k_misfit<T><<<kMisfitBlocks, 256, 0, st>>>(tr, obs, ntr, dmis + 1);
+  k_misfit_sum<<<1, 1, 0, st>>>(dmis + 1, dmis);
   // ---- adjoint sweep ----
   AdjArgs<T> A;
-  A.nx = c.nx; A.nz = c.nz; A.nsls = N; A.kind = c.medium; A.fs = c.free_surface;
-  A.Lx = p->Lx; A.Rx = p->Rx; A.Tz = p->Tz; A.Bz = p->Bz; A.wx = p->wx; A.hz = p->hz;
+  A.nx = c.nx; A.nz = c.nz; A.ld = ld; A.fs = c.free_surface;
+  A.Lx = p->Lx; A.Rx = p->Rx; A.Tz = p->Tz; A.Bz = p->Bz; A.wx = p->wx;
   A.dt = (T)c.dt;
   for (int k = 0; k < 4; ++k) {
     A.Dx[k] = (T)(kD8[k] / c.dx);
@@ -1187,32 +1571,89 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
     A.a1[n] = a.a1[n];
     A.a2[n] = a.a2[n];
   }
-  A.rho = (const T *)m->rho; A.c11 = (const T *)m->c11; A.c13 = (const T *)m->c13;
-  A.c33 = (const T *)m->c33; A.c55 = (const T *)m->c55; A.tau = (const T *)m->tau;
-  A.c15 = (const T *)m->c15; A.c35 = (const T *)m->c35;
+  A.rho = a.rho; A.c11 = a.c11; A.c13 = a.c13; A.c33 = a.c33; A.c55 = a.c55; A.tau = a.tau;
+  A.c15 = a.c15; A.c35 = a.c35;
   A.tx = (const T *)p->tabx; A.tz = (const T *)p->tabz;
-  A.np = np; A.psix_plane = p->psix_plane; A.psiz_plane = p->psiz_plane;
+  A.np = np; A.psix_plane = px; A.psiz_plane = pz;
+  A.keep_bar = l2_hints_fit(8LL * np * (long long)sizeof(T), p->l2_bytes);
   Slot<T> ab = mk(adj);
   if ((rc = cuda_check(cudaMemsetAsync(adj, 0, sbytes, st), "zero adjoint"))) return rc;
-  if ((rc = cuda_check(cudaMemsetAsync(rbar, 0, 7 * np * sizeof(T), st), "zero scratch"))) return rc;
-  if (tti && (rc = cuda_check(cudaMemsetAsync(teb, 0, 5 * np * sizeof(T), st), "zero TTI scratch"))) return rc;
-  if (!accumulate)
-    if ((rc = cuda_check(cudaMemsetAsync(grad, 0, 8 * np * sizeof(double), st), "zero gradient"))) return rc;
-  double *gr = grad, *g11 = grad + np, *g13 = grad + 2 * np, *g33 = grad + 4 * np;
-  double *g55 = grad + 6 * np, *gt = grad + 7 * np, *g15 = grad + 3 * np, *g35 = grad + 5 * np;
-  const dim3 blk(32, 8);
-  const dim3 gU((c.nx - 2 * L + 31) / 32, (c.nz - 2 * L + 7) / 8);
-  const dim3 gA((c.nx + 31) / 32, (c.nz + 7) / 8);
-  // 4-cell forms of the transposed derivatives where the planes allow
-  // 128-bit access (the same condition as the split pair)
-  const bool vec4 = split_ok;
-  const dim3 gU4(((c.nx - 2 * L) / 4 + 31) / 32, (c.nz - 2 * L + 7) / 8);
-  const dim3 gA4((c.nx / 4 + 31) / 32, (c.nz + 7) / 8);
-  int lrc = VI_OK;  // first launch error of the adjoint sweep
-  auto lc = [&](auto kernel, dim3 g, dim3 b, auto... args) {
-    const cudaError_t e = launch_pdl(kernel, g, b, 0, st, true, args...);
-    if (e != cudaSuccess && !lrc) lrc = cuda_check(e, "adjoint launch");
+  if ((rc = cuda_check(cudaMemsetAsync(rbar, 0, (char *)pmed - (char *)rbar, st), "zero scratch"))) return rc;
+  // TMA maps: the planes' and accumulators' places do not change over the sweep
+  const int e = (int)sizeof(T), ntx = fxa.ntx, nslots = keep_all ? nt + 1 : K + 1;
+  constexpr int TX = AG::TX, TZ = AG::TZ, WX = AG::WX, HZ = AG::HZ, WC = AG::WC;
+  const int acc0 = ACC_TAU, nacc = acc_planes(c.medium) - acc0;
+  double *const acck = acc + acc0 * np;
+  AdjMaps ms_s{}, ms_v{}, ms_t{};  // k_adj_stress / k_adj_sigma_tti, k_adj_vel, k_adj_stress_tti
+  auto em = [&](CUtensorMap *map, const void *base, int es, int depth, int bx, int bz, int bd) {
+    if (!rc) rc = encode_map(map, base, es, ld, c.nz, depth, np, bx, bz, bd);
   };
+  auto es4 = [&](CUtensorMap *map, int bx, int bz) {
+    if (!rc) rc = encode_map_slots(map, seg, e, ld, c.nz, 5, np, nslots, slot, bx, bz);
+  };
+  rc = VI_OK;
+  em(&ms_s.px, dbar, e, 4, WX, TZ, 1);
+  em(&ms_s.pz, dbar, e, 4, TX, HZ, 1);
+  es4(&ms_s.st_a, WX, HZ);
+  em(&ms_s.own, ab.sxx(), e, 3, TX, TZ, 3);
+  em(&ms_v.px, rbar, e, 4, WX, TZ, 1);
+  em(&ms_v.pz, rbar, e, 4, TX, HZ, 1);
+  es4(&ms_v.st_a, WX, TZ);
+  es4(&ms_v.st_b, WX, HZ);
+  es4(&ms_v.st_c, TX, HZ);
+  em(&ms_v.own, ab.vx(), e, 2, TX, TZ, 2);
+  em(&ms_v.acc, acc, 8, 2, TX, TZ, 2);
+  if (tti) {
+    em(&ms_t.px, fe, e, 3, WX, TZ + 2, 3);
+    em(&ms_t.pz, ab.sxx(), e, 3, WX, TZ + 2, 3);
+    em(&ms_t.cc, a.c55, e, 1, WC, TZ + 1, 1);
+    em(&ms_t.c2, a.c15, e, 1, WX, TZ + 2, 1);
+    em(&ms_t.c3, a.c35, e, 1, WX, TZ + 2, 1);
+    em(&ms_t.acc, acck, 8, nacc, TX, TZ, nacc);
+  } else {
+    if (N > 0) em(&ms_s.mem, ab.m(), e, 3 * N, TX, TZ, 3 * N);
+    em(&ms_s.cc, a.c55, e, 1, WC, TZ + 1, 1);
+    em(&ms_s.acc, acck, 8, nacc, TX, TZ, nacc);
+  }
+  if (rc) return rc;
+  int lrc = VI_OK;  // first launch error of the adjoint sweep
+  bool opt_in = true;  // the first call per kernel only opts into its dynamic shared memory
+  auto lc = [&](auto kernel, int smem, auto... args) {
+    if (lrc) return;
+    const cudaError_t err = opt_in ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
+                                   : launch_pdl(kernel, dim3(antiles), dim3(AG::NT), (size_t)smem, st, true, args...);
+    if (err != cudaSuccess) lrc = cuda_check(err, "adjoint launch");
+  };
+  int *const derr = (int *)p->errflag;
+  auto stress_t = [&](auto n, const Slot<T> &x0, int sl) {
+    constexpr int NN = decltype(n)::value;
+    if (tti) {
+      lc(k_adj_sigma_tti<T, NN>, SigmaTtiSmem<T>::SIZE, A, ms_s, x0, sl, ntx, ab.sxx(), fe, derr);
+      lc(k_adj_stress_tti<T, NN>, TtiSmem<T>::SIZE, A, ms_t, ntx, (const T *)fe, ab.m(), ab.psix(), ab.psiz(), rbar,
+         acck, derr);
+    } else if (c.medium == VI_MEDIUM_ISO) {
+      lc(k_adj_stress<T, VI_MEDIUM_ISO, NN>, StressK<T, VI_MEDIUM_ISO, NN>::S::SIZE, A, ms_s, x0, sl, ntx, ab.sxx(),
+         ab.m(), ab.psix(), ab.psiz(), rbar, acck, derr);
+    } else {
+      lc(k_adj_stress<T, VI_MEDIUM_VTI, NN>, StressK<T, VI_MEDIUM_VTI, NN>::S::SIZE, A, ms_s, x0, sl, ntx, ab.sxx(),
+         ab.m(), ab.psix(), ab.psiz(), rbar, acck, derr);
+    }
+  };
+  auto reverse_step = [&](const Slot<T> &x0, const Slot<T> &x1, int sl, int it) {
+    switch (N) {
+      case 0: stress_t(std::integral_constant<int, 0>{}, x0, sl); break;
+      case 1: stress_t(std::integral_constant<int, 1>{}, x0, sl); break;
+      case 2: stress_t(std::integral_constant<int, 2>{}, x0, sl); break;
+      case 3: stress_t(std::integral_constant<int, 3>{}, x0, sl); break;
+      case 4: stress_t(std::integral_constant<int, 4>{}, x0, sl); break;
+      default: stress_t(std::integral_constant<int, 5>{}, x0, sl); break;
+    }
+    fxa.it = it;
+    lc(k_adj_vel<T>, VelSmem<T>::SIZE, A, ms_v, x0, x1, sl, fxa, obs, ab.vx(), ab.psix(), ab.psiz(), dbar, acc);
+  };
+  reverse_step(ab, ab, 0, 0);
+  opt_in = false;
+  if (lrc) return lrc;
   // keep_all: one segment of nt steps whose states are all kept
   for (int qseg = keep_all ? 0 : nck - 1; qseg >= 0; --qseg) {
     const int s0 = keep_all ? 0 : qseg * K, s1 = keep_all ? nt : std::min(nt, s0 + K);
@@ -1223,74 +1664,23 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
       return rc;
     NvtxRange nr_seg("vi_gradient: segment recompute and adjoint");
     for (int k = 0; !keep_all && k < s1 - s0; ++k) {
-      T *nxt = seg + (size_t)(k + 1) * slot;
-      if (use_split) {
-        // straight from slot k into slot k + 1 (no copy of the state)
-        const Slot<T> out = mk(nxt);
-        if ((rc = fwd_step(mk(seg + (size_t)k * slot), s0 + k, nullptr, k > 0, &out))) return rc;
-      } else {
-        if ((rc = cuda_check(cudaMemcpyAsync(nxt, seg + (size_t)k * slot, sbytes, cudaMemcpyDeviceToDevice, st),
-                             "segment copy")))
-          return rc;
-        if ((rc = fwd_step(mk(nxt), s0 + k, nullptr, false))) return rc;
-      }
+      // straight from slot k into slot k + 1 (no copy of the state)
+      const Slot<T> out = mk(seg + (size_t)(k + 1) * slot);
+      if ((rc = fwd_step(mk(seg + (size_t)k * slot), s0 + k, nullptr, k > 0, &out))) return rc;
       if ((rc = yield(1))) return rc;
     }
     for (int it = s1 - 1; it >= s0; --it) {
       const Slot<T> x0 = mk(seg + (size_t)(it - s0) * slot), x1 = mk(seg + (size_t)(it - s0 + 1) * slot);
       // every kernel of the step overlaps its predecessor's tail and waits
       // for it at entry (programmatic dependent launch)
-      if (c.free_surface) lc(k_mirror_t<T>, dim3((c.nx + 127) / 128), dim3(128), ab.szz(), ab.sxz(), c.nx);
-      if (tti) {
-        const dim3 gS((c.nx - 2 * L + 127) / 128);
-        switch (N) {
-          case 0: lc(k_tti_fwd_rates<T, 0>, gU, blk, A, x0, x1, pscr); break;
-          case 1: lc(k_tti_fwd_rates<T, 1>, gU, blk, A, x0, x1, pscr); break;
-          case 2: lc(k_tti_fwd_rates<T, 2>, gU, blk, A, x0, x1, pscr); break;
-          case 3: lc(k_tti_fwd_rates<T, 3>, gU, blk, A, x0, x1, pscr); break;
-          case 4: lc(k_tti_fwd_rates<T, 4>, gU, blk, A, x0, x1, pscr); break;
-          default: lc(k_tti_fwd_rates<T, 5>, gU, blk, A, x0, x1, pscr); break;
-        }
-        if (c.free_surface) lc(k_tti_fwd_surface<T>, gS, dim3(128), A, pscr);
-        lc(k_tti_ebar_t<T>, gU, blk, A, ab, (const T *)pscr, teb, q, tq15, tq35, g11, g13, g15, g33, g35);
-        if (c.free_surface) lc(k_tti_surface_t<T>, gS, dim3(128), A, (const T *)pscr, teb, g13, g33, g35);
-        switch (N) {
-          case 0: lc(k_tti_stress_t<T, 0>, gU, blk, A, ab, (const T *)pscr, (const T *)teb, rbar, gt); break;
-          case 1: lc(k_tti_stress_t<T, 1>, gU, blk, A, ab, (const T *)pscr, (const T *)teb, rbar, gt); break;
-          case 2: lc(k_tti_stress_t<T, 2>, gU, blk, A, ab, (const T *)pscr, (const T *)teb, rbar, gt); break;
-          case 3: lc(k_tti_stress_t<T, 3>, gU, blk, A, ab, (const T *)pscr, (const T *)teb, rbar, gt); break;
-          case 4: lc(k_tti_stress_t<T, 4>, gU, blk, A, ab, (const T *)pscr, (const T *)teb, rbar, gt); break;
-          default: lc(k_tti_stress_t<T, 5>, gU, blk, A, ab, (const T *)pscr, (const T *)teb, rbar, gt); break;
-        }
-      } else switch (N) {
-        case 0: lc(k_stress_t<T, 0>, gU, blk, A, x0, x1, ab, rbar, q, g11, g13, g33, gt); break;
-        case 1: lc(k_stress_t<T, 1>, gU, blk, A, x0, x1, ab, rbar, q, g11, g13, g33, gt); break;
-        case 2: lc(k_stress_t<T, 2>, gU, blk, A, x0, x1, ab, rbar, q, g11, g13, g33, gt); break;
-        case 3: lc(k_stress_t<T, 3>, gU, blk, A, x0, x1, ab, rbar, q, g11, g13, g33, gt); break;
-        case 4: lc(k_stress_t<T, 4>, gU, blk, A, x0, x1, ab, rbar, q, g11, g13, g33, gt); break;
-        default: lc(k_stress_t<T, 5>, gU, blk, A, x0, x1, ab, rbar, q, g11, g13, g33, gt); break;
-      }
-      if (vec4)
-        lc(k_rates_t4<T>, gU4, blk, A, ab, (const T *)rbar);
-      else
-        lc(k_rates_t<T>, gU, blk, A, ab, (const T *)rbar);
-      lc(k_residual<T>, dim3((nrec + 127) / 128), dim3(128), ab, x1, (const int2 *)p->drec, nrec, obs, nt, it, c.nx);
-      lc(k_vel_t<T>, gU, blk, A, x0, ab, rbar, h);  // the 4-cell form measured slower
-      if (shot->nsrc > 0)
-        lc(k_force_rho_t<T>, dim3((shot->nsrc + 127) / 128), dim3(128), A, ab, (const int4 *)p->dsrc,
-           (const T *)p->damp, shot->nsrc, (const T *)shot->wavelet_dev, shot->wavelet_nt, it, h);
-      lc(k_gather<T>, gA, blk, (const T *)h, gr, (const T *)q, g55, c.nx, c.nz);
-      if (tti) lc(k_tti_gather<T>, gA, blk, (const T *)tq15, (const T *)tq35, g15, g35, c.nx, c.nz);
-      if (vec4)
-        lc(k_div_t4<T>, gA4, blk, A, ab, (const T *)rbar);
-      else
-        lc(k_div_t<T>, gA, blk, A, ab, (const T *)rbar);
+      reverse_step(x0, x1, it - s0, it);
       if (lrc) return lrc;
       if ((rc = yield(2))) return rc;
     }
   }
   if (lrc) return lrc;
-  if (c.medium == VI_MEDIUM_ISO) k_fold_iso<<<(unsigned)((np + 255) / 256), 256, 0, st>>>(np, grad);
+  k_adj_finish<<<dim3((c.nx + 31) / 32, (c.nz + 7) / 8), dim3(32, 8), 0, st>>>(c.medium, c.nx, c.nz, ld, (double)A.dt,
+                                                                              acc, accumulate, grad);
   p->last_kernel = 1;
   if ((rc = cuda_check(cudaGetLastError(), "gradient launch"))) return rc;
   if ((rc = cuda_check(cudaMemcpyAsync(misfit, dmis, sizeof(double), cudaMemcpyDeviceToHost, st), "misfit")))

@@ -941,4 +941,23 @@ int encode_map(CUtensorMap *map, const void *base, int esize, int nx, int nz, lo
   return VI_OK;
 }
 
+// Map of `planes` planes (stride plane_stride elements) in each of `slots`
+// slots (stride slot_stride elements): coordinates column, row, plane, slot; a
+// box is box_x x box_z cells of one plane.
+int encode_map_slots(CUtensorMap *map, const void *base, int esize, int nx, int nz, int planes, long long plane_stride,
+                     int slots, long long slot_stride, int box_x, int box_z) {
+  auto fn = encoder();
+  if (!fn) return set_error(VI_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  cuuint64_t dims[4] = {(cuuint64_t)nx, (cuuint64_t)nz, (cuuint64_t)planes, (cuuint64_t)slots};
+  cuuint64_t strides[3] = {(cuuint64_t)nx * esize, (cuuint64_t)plane_stride * esize, (cuuint64_t)slot_stride * esize};
+  cuuint32_t box[4] = {(cuuint32_t)box_x, (cuuint32_t)box_z, 1, 1};
+  cuuint32_t es[4] = {1, 1, 1, 1};
+  CUresult r = fn(map, esize == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,
+                  const_cast<void *>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return set_error(VI_ERR_ARG, "cuTensorMapEncodeTiled failed (code " + std::to_string((int)r) + ")");
+  return VI_OK;
+}
+
 }  // namespace vb

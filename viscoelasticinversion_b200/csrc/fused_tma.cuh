@@ -156,5 +156,7 @@ int encode_parity(TmaMaps &m, const TmaBoxes &b, const vi_config &c, T *const in
 // Encodes a 2D (depth = 1) or 3D tensor map over an x-fastest array.
 int encode_map(CUtensorMap *map, const void *base, int esize, int nx, int nz, long long depth,
                long long plane_stride_elems, int box_x, int box_z, int box_d);
+int encode_map_slots(CUtensorMap *map, const void *base, int esize, int nx, int nz, int planes, long long plane_stride,
+                     int slots, long long slot_stride, int box_x, int box_z);
 
 }  // namespace vb

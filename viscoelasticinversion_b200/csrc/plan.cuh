@@ -46,6 +46,7 @@ struct vi_plan {
   // forward_host buffers and the gradient's workspace (device, grown on demand)
   void *fwd = nullptr;
   size_t fwd_bytes = 0;
+  size_t device_bytes = 0;  // of device memory in all, once a gradient has asked
   // layout of the gradient's kept states whose never-written cells are
   // known zero (0: none)
   unsigned long long grad_zero_key = 0;

@@ -139,7 +139,12 @@ int64_t footprint(const vi_request &r) {
     while (K * K < r.nt) ++K;
     const int64_t nck = (r.nt + K - 1) / K;
     const int64_t slot = ns * np * e + psi / 2;
-    b += (nck + K + 2) * slot + 13 * np * e + 8 * np * 8 + tr;
+    // adjoint scratch: rbar, dbar, TTI's effective rates, odd rows' medium copy
+    // and the FP64 accumulators; what the forward-only planes above leave over
+    // (second state copy, spare) counts towards it
+    const bool tti = c.medium == VI_MEDIUM_TTI;
+    const int64_t scratch = (8 + (tti ? 6 : 0) + (c.nx % 4 != 0 ? 8 : 0)) * np * e + (tti ? 11 : 7) * np * 8;
+    b += (nck + K + 2) * slot + std::max(13 * np * e, scratch - (2 * ns + 6) * np * e) + 8 * np * 8 + tr;
   }
   return b;
 }

@@ -503,6 +503,19 @@ __global__ void __launch_bounds__(256) k_copy_planes(const __grid_constant__ Pad
   }
 }
 
+template <typename T>
+int copy_planes(const T *const *src, T *const *dst, int n, int lds, int ldd, int nx, int nz, cudaStream_t st) {
+  PadPlanes<T> pl;
+  for (int q = 0; q < n; ++q) {
+    pl.src[q] = src[q];
+    pl.dst[q] = dst[q];
+  }
+  k_copy_planes<T><<<dim3((nx + 127) / 128, (nz + 7) / 8, n), 256, 0, st>>>(pl, lds, ldd, 0, nx, 0, 0, nz);
+  return cuda_check(cudaGetLastError(), "copy planes launch");
+}
+template int copy_planes<float>(const float *const *, float *const *, int, int, int, int, int, cudaStream_t);
+template int copy_planes<double>(const double *const *, double *const *, int, int, int, int, int, cudaStream_t);
+
 // The split pair for rows that are no multiple of 4 cells, or planes off a
 // 16-byte boundary: state and medium are copied once per call into planes of
 // the plan whose rows start on 16-byte boundaries, stepped there, and the

@@ -131,6 +131,9 @@ template <typename T>
 int split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st,
                 int mode);
 
+// n planes of nx x nz cells (at most 28) from row stride lds to ldd.
+template <typename T>
+int copy_planes(const T *const *src, T *const *dst, int n, int lds, int ldd, int nx, int nz, cudaStream_t st);
 // The same steps for rows and planes the split kernels cannot take as they
 // are (nx % 4 != 0, unaligned planes), on copies laid out by the plan.
 template <typename T>

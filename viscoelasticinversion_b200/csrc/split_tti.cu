@@ -315,15 +315,18 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
     keep_edge4(sxz, xe - gi0, a.sxz + g);
   }
   if (!finite3(sxx, szz, sxz)) atomicOr(x.err, kErrNonFinite);
-  // sigma is re-read by the next velocity pass: keep it in L2
-  sth4(a.sxx + g, sxx, l2_keep_c<HINT>());
-  sth4(a.szz + g, szz, l2_keep_c<HINT>());
-  sth4(a.sxz + g, sxz, l2_keep_c<HINT>());
+  // sigma is re-read by the next velocity pass: keep it in L2 (the gradient's
+  // sweeps write it to another slot)
+  T *const osxx = a.sxx_o ? a.sxx_o : a.sxx, *const oszz = a.sxx_o ? a.szz_o : a.szz;
+  T *const osxz = a.sxx_o ? a.sxz_o : a.sxz;
+  sth4(osxx + g, sxx, l2_keep_c<HINT>());
+  sth4(oszz + g, szz, l2_keep_c<HINT>());
+  sth4(osxz + g, sxz, l2_keep_c<HINT>());
   if (x.fs == kFsImaging) {
     // stress images: szz(L-k) = -szz(L+k), k = 1..4; sxz(L-1-k) = -sxz(L+k), k = 0..3
     const int k = gj - L;
-    if (k >= 1 && k <= L) stg4(a.szz + (long long)(L - k) * ld + gi0, mul4(splat4<T>(T(-1)), szz));
-    if (k >= 0 && k < L) stg4(a.sxz + (long long)(L - 1 - k) * ld + gi0, mul4(splat4<T>(T(-1)), sxz));
+    if (k >= 1 && k <= L) stg4(oszz + (long long)(L - k) * ld + gi0, mul4(splat4<T>(T(-1)), szz));
+    if (k >= 0 && k < L) stg4(osxz + (long long)(L - 1 - k) * ld + gi0, mul4(splat4<T>(T(-1)), sxz));
   }
 }
 
