@@ -593,6 +593,7 @@ extern "C" int vi_batch_create(const vi_config *cfgs, int32_t nshots, vi_batch *
       vi_batch_destroy(b);
       return rc;
     }
+    b->plans[i]->no_resident = true;  // shots run side by side
     b->afda |= cfgs[i].free_surface == kFsAfda;
   }
   b->med.assign(nshots, vi_medium{});

@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -46,6 +47,41 @@ int ensure_buffer(vi_plan *p, void **buf, size_t *have, size_t need) {
   *have = need;
   p->bytes += need;
   return VI_OK;
+}
+
+// Plans of this process, for others_in_flight.  Only which of two bitwise equal
+// forms of the step runs depends on it.
+static std::mutex g_plans_mu;
+static std::vector<vi_plan *> g_plans;
+
+bool others_in_flight(const vi_plan *p) {
+  std::lock_guard<std::mutex> lk(g_plans_mu);
+  for (vi_plan *q : g_plans) {
+    if (q == p || q->device != p->device) continue;
+    if (q->in_call) return true;
+    if (!q->done_pending) continue;
+    if (cudaEventQuery(q->done) == cudaErrorNotReady) {
+      cudaGetLastError();
+      return true;
+    }
+    q->done_pending = false;
+  }
+  return false;
+}
+
+void mark_steps(vi_plan *p, cudaStream_t st) {
+  std::lock_guard<std::mutex> lk(g_plans_mu);
+  if (!p->done && cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    p->done = nullptr;
+    return;
+  }
+  p->done_pending = cudaEventRecord(p->done, st) == cudaSuccess;
+}
+
+void mark_call(vi_plan *p, bool running) {
+  std::lock_guard<std::mutex> lk(g_plans_mu);
+  p->in_call = running;
 }
 
 // CPML profile of CPML.jl:91-189 evaluated at integer (half=0) or half
@@ -458,7 +494,9 @@ static int step_impl(vi_plan *p, const vi_medium *m, vi_fields *f, const vi_shot
     // the one-tile-per-CTA pair measures faster than the pipelined pair on
     // B200 (2048 x 1024 VTI: 27.6 vs 24.4 Gpt/s), so it is the default
     const int mode = variant == 6 ? kSplitPipelined : variant == 8 ? kSplitLdg : kSplitVelTma;
-    rc = split_steps<T>(p, a, s, it0, nsteps, st, mode);
+    rc = VI_ERR_BUDGET;
+    if (variant == 0 && resident_eligible_cfg(p, nsteps)) rc = resident_steps<T>(p, a, s, it0, nsteps, st);
+    if (rc == VI_ERR_BUDGET) rc = split_steps<T>(p, a, s, it0, nsteps, st, mode);
     if (rc) return rc;
     p->last_kernel = variant == 0 ? 5 : variant;
   } else {
@@ -481,6 +519,7 @@ static int step_impl(vi_plan *p, const vi_medium *m, vi_fields *f, const vi_shot
                                      p->nsm, st)))
       return rc;
   }
+  if (nsteps >= kResidentMinSteps) mark_steps(p, st);
   return cuda_check(cudaGetLastError(), "step launch");
 }
 
@@ -555,6 +594,10 @@ extern "C" int vi_plan_create(const vi_config *cfg, vi_plan **out) {
   if (rc) goto fail;
   rc = cuda_check(cudaDeviceSynchronize(), "plan create");
   if (rc) goto fail;
+  {
+    std::lock_guard<std::mutex> lk(g_plans_mu);
+    g_plans.push_back(p);
+  }
   *out = p;
   return VI_OK;
 fail:
@@ -576,8 +619,13 @@ extern "C" int vi_plan_destroy(vi_plan *p) {
   int prev = 0;
   cudaGetDevice(&prev);
   cudaSetDevice(p->device);
+  {
+    std::lock_guard<std::mutex> lk(g_plans_mu);
+    g_plans.erase(std::remove(g_plans.begin(), g_plans.end(), p), g_plans.end());
+    if (p->done) cudaEventDestroy(p->done);
+  }
   void *bufs[] = {p->psix, p->psiz, p->tabx, p->tabz, p->scratch, p->alt, p->slo,
-                  p->dsrc, p->damp, p->drec, p->tile_lists, p->fwd, p->errflag, p->wave_ctl, p->pad};
+                  p->dsrc, p->damp, p->drec, p->tile_lists, p->fwd, p->errflag, p->wave_ctl, p->pad, p->shadow};
   for (void *b : bufs)
     if (b) cudaFree(b);
   cudaSetDevice(prev);

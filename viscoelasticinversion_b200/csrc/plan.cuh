@@ -23,6 +23,17 @@ struct vi_plan {
   void *tabx = nullptr, *tabz = nullptr;  // 6*nx and 6*nz reals
   void *scratch = nullptr;                // plain path: 6 planes
   void *alt = nullptr;                    // fused path: second v/sigma copy (5 planes)
+  // the plan's steps share the GPU with other streams' (batches, the server):
+  // the default step then never takes the whole chip (resident.cu)
+  bool no_resident = false;
+  // whether work of this plan may still run: recorded after each longer step
+  // call, in_call during a gradient (both under capi.cu's list of plans)
+  cudaEvent_t done = nullptr;
+  bool done_pending = false, in_call = false;
+  // resident steps: the tiles' edges beside the pass that wrote them
+  void *shadow = nullptr;
+  size_t shadow_bytes = 0;
+  unsigned shadow_pass = 1;
   // split step on grids whose rows need padding: state, medium, TTI's
   // second memory-variable set (grown on demand)
   void *pad = nullptr;
@@ -62,6 +73,12 @@ struct vi_plan {
 
 namespace vb {
 int set_error(int code, const std::string &msg);
+// Whether another plan of this process has steps or a gradient in flight on the
+// device (the resident step, which takes whole SMs, then leaves it to kernels
+// that run side by side); marks for this plan.
+bool others_in_flight(const vi_plan *p);
+void mark_steps(vi_plan *p, cudaStream_t st);
+void mark_call(vi_plan *p, bool running);
 int cuda_check(cudaError_t e, const char *what);
 // Grow-only device buffer.
 int ensure_buffer(vi_plan *p, void **buf, size_t *have, size_t need);

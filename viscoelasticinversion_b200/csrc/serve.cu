@@ -196,7 +196,9 @@ int take_plan(vi_server *s, const vi_config &c, vi_plan **out) {
       }
     }
   }
-  return vi_plan_create(&c, out);
+  const int rc = vi_plan_create(&c, out);
+  if (!rc) (*out)->no_resident = true;  // requests run side by side
+  return rc;
 }
 
 // Keeps a finished request's plan for reuse (oldest evicted beyond the cap).

@@ -149,6 +149,18 @@ bool wave_eligible_cfg(const vi_config &c);
 template <typename T>
 int wave_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st);
 
+// The same steps as one cooperative kernel that keeps the grid on the chip
+// (resident.cu): ISO/VTI, imaging or no surface, FP32 or FP64.  Bitwise equal
+// to split_steps.  Returns VI_ERR_BUDGET, having done nothing, when the device
+// cannot hold the launch.
+// From 16 steps on (256 x 256 VTI FP32: 107 us against 160 for the pair; 512 x
+// 512 174 against 202; about 40 us of loading, launching and storing are won
+// back in some 5 steps).
+constexpr int kResidentMinSteps = 16;
+bool resident_eligible_cfg(const vi_plan *p, int nsteps);
+template <typename T>
+int resident_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st);
+
 // true when split_steps can run this plan and these pointers
 template <typename T>
 bool split_eligible(const vi_plan *p, const StepArgs<T> &a);
