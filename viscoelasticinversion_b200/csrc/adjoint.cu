@@ -1697,13 +1697,13 @@ extern "C" int vi_gradient(vi_plan *p, const vi_medium *med_dev, const vi_shot *
                            double *grad_dev, double *misfit_host, void *stream) {
   if (!p || !misfit_host) return set_error(VI_ERR_ARG, "gradient: NULL argument");
   cudaStream_t st = (cudaStream_t)stream;
-  mark_call(p, true);
+  if (!p->no_resident) mark_call(p, true);
   const int rc = p->cfg.precision == VI_F64
                      ? gradient_impl<double>(p, med_dev, shot, nt, (const double *)obs_dev, checkpoint_every,
                                              accumulate, grad_dev, misfit_host, st)
                      : gradient_impl<float>(p, med_dev, shot, nt, (const float *)obs_dev, checkpoint_every,
                                             accumulate, grad_dev, misfit_host, st);
-  mark_call(p, false);
+  if (!p->no_resident) mark_call(p, false);
   return rc;
 }
 

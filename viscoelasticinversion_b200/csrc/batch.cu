@@ -657,7 +657,9 @@ extern "C" int vi_batch_run(vi_batch *b, int32_t flags, void *stream) {
   if (!b) return set_error(VI_ERR_ARG, "batch is NULL");
   NvtxRange nr("vi_batch_run");
   cudaStream_t st = (cudaStream_t)stream;
-  return b->precision == VI_F64 ? run_impl<double>(b, flags, st) : run_impl<float>(b, flags, st);
+  const int rc = b->precision == VI_F64 ? run_impl<double>(b, flags, st) : run_impl<float>(b, flags, st);
+  if (!rc && b->n > 0) mark_steps(b->plans[0], st);  // the run's end on st is every shot's
+  return rc;
 }
 
 extern "C" int vi_batch_status(vi_batch *b, void *stream, int32_t *kernel_form) {

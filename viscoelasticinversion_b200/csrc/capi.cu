@@ -318,6 +318,17 @@ static bool in_update_region(const vi_config &c, int i, int j) {
   return i >= L && i < c.nx - L && j >= L && j < c.nz - L;
 }
 
+// Whether the device list holds these entries already (it is then left alone,
+// and the call does not wait for the stream); the record of what it holds.
+template <typename E>
+static bool staged(const std::vector<char> &have, const std::vector<E> &v) {
+  return !v.empty() && have.size() == v.size() * sizeof(E) && std::memcmp(have.data(), v.data(), have.size()) == 0;
+}
+template <typename E>
+static void keep(std::vector<char> &have, const std::vector<E> &v) {
+  have.assign((const char *)v.data(), (const char *)v.data() + v.size() * sizeof(E));
+}
+
 // Copies the shot's source / receiver lists to the plan's device buffers.
 template <typename T>
 int stage_shot(vi_plan *p, const vi_shot *s, cudaStream_t st) {
@@ -339,6 +350,7 @@ int stage_shot(vi_plan *p, const vi_shot *s, cudaStream_t st) {
     }
     if (s->nsrc > p->src_cap) {
       size_t h1 = 0, h2 = 0;
+      p->src_host.clear();
       if (p->dsrc) { cudaFree(p->dsrc); p->bytes -= (size_t)p->src_cap * sizeof(int4); p->dsrc = nullptr; }
       if (p->damp) { cudaFree(p->damp); p->bytes -= (size_t)p->src_cap * sizeof(double); p->damp = nullptr; }
       int rc = ensure_buffer(p, &p->dsrc, &h1, (size_t)s->nsrc * sizeof(int4));
@@ -347,15 +359,20 @@ int stage_shot(vi_plan *p, const vi_shot *s, cudaStream_t st) {
       if (rc) return rc;
       p->src_cap = s->nsrc;
     }
-    int rc = cuda_check(cudaMemcpyAsync(p->dsrc, hs.data(), hs.size() * sizeof(int4),
-                                        cudaMemcpyHostToDevice, st), "copy sources");
-    if (rc) return rc;
-    rc = cuda_check(cudaMemcpyAsync(p->damp, ha.data(), ha.size() * sizeof(T),
-                                    cudaMemcpyHostToDevice, st), "copy amplitudes");
-    if (rc) return rc;
-    // the staging vectors die at return: wait for the pageable copies
-    rc = cuda_check(cudaStreamSynchronize(st), "stage sources");
-    if (rc) return rc;
+    if (!staged(p->src_host, hs) || !staged(p->amp_host, ha)) {
+      p->src_host.clear();
+      int rc = cuda_check(cudaMemcpyAsync(p->dsrc, hs.data(), hs.size() * sizeof(int4),
+                                          cudaMemcpyHostToDevice, st), "copy sources");
+      if (rc) return rc;
+      rc = cuda_check(cudaMemcpyAsync(p->damp, ha.data(), ha.size() * sizeof(T),
+                                      cudaMemcpyHostToDevice, st), "copy amplitudes");
+      if (rc) return rc;
+      // the staging vectors die at return: wait for the pageable copies
+      rc = cuda_check(cudaStreamSynchronize(st), "stage sources");
+      if (rc) return rc;
+      keep(p->src_host, hs);
+      keep(p->amp_host, ha);
+    }
   }
   if (s->nrec > 0) {
     if (!s->rec_host) return set_error(VI_ERR_ARG, "receivers need rec_host");
@@ -368,16 +385,21 @@ int stage_shot(vi_plan *p, const vi_shot *s, cudaStream_t st) {
     }
     if (s->nrec > p->rec_cap) {
       size_t h1 = 0;
+      p->rec_host.clear();
       if (p->drec) { cudaFree(p->drec); p->bytes -= (size_t)p->rec_cap * sizeof(int2); p->drec = nullptr; }
       int rc = ensure_buffer(p, &p->drec, &h1, (size_t)s->nrec * sizeof(int2));
       if (rc) return rc;
       p->rec_cap = s->nrec;
     }
-    int rc = cuda_check(cudaMemcpyAsync(p->drec, hr.data(), hr.size() * sizeof(int2),
-                                        cudaMemcpyHostToDevice, st), "copy receivers");
-    if (rc) return rc;
-    rc = cuda_check(cudaStreamSynchronize(st), "stage receivers");
-    if (rc) return rc;
+    if (!staged(p->rec_host, hr)) {
+      p->rec_host.clear();
+      int rc = cuda_check(cudaMemcpyAsync(p->drec, hr.data(), hr.size() * sizeof(int2),
+                                          cudaMemcpyHostToDevice, st), "copy receivers");
+      if (rc) return rc;
+      rc = cuda_check(cudaStreamSynchronize(st), "stage receivers");
+      if (rc) return rc;
+      keep(p->rec_host, hr);
+    }
   }
   return VI_OK;
 }
@@ -519,7 +541,9 @@ static int step_impl(vi_plan *p, const vi_medium *m, vi_fields *f, const vi_shot
                                      p->nsm, st)))
       return rc;
   }
-  if (nsteps >= kResidentMinSteps) mark_steps(p, st);
+  // (a batch marks its runs, the server its requests: an event per shot would
+  // cost a new batch 20 ms)
+  if (nsteps >= kResidentMinSteps && !p->no_resident) mark_steps(p, st);
   return cuda_check(cudaGetLastError(), "step launch");
 }
 

@@ -12,6 +12,8 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <cstring>
+#include <utility>
 #include <vector>
 
 #include "fused.cuh"
@@ -378,13 +380,14 @@ void build_tile_lists(int nx, int nz, int TX, int TZ, int HV, const vi_shot *s,
   ntx = (nx - 2 * L + TX - 1) / TX;
   ntz = (nz - 2 * L + TZ - 1) / TZ;
   const int ntiles = ntx * ntz;
-  std::vector<std::vector<int4>> per(ntiles);
+  std::vector<std::pair<int, int4>> all;  // (tile, entry)
   auto own_tile = [&](int i, int j) { return ((j - L) / TZ) * ntx + (i - L) / TX; };
   if (s) {
+    all.reserve((size_t)s->nsrc + s->nrec);
     for (int q = 0; q < s->nsrc; ++q) {
       const vi_source &v = s->src_host[q];
       if (v.kind == VI_SRC_EXPLOSIVE) {
-        per[own_tile(v.i, v.j)].push_back(make_int4(v.i, v.j, q, TL_EXPLOSIVE));
+        all.emplace_back(own_tile(v.i, v.j), make_int4(v.i, v.j, q, TL_EXPLOSIVE));
         continue;
       }
       const int kind = v.kind == VI_SRC_FORCE_X ? TL_FORCE_X : TL_FORCE_Z;
@@ -394,44 +397,56 @@ void build_tile_lists(int nx, int nz, int TX, int TZ, int HV, const vi_shot *s,
         for (int bx = bx0 < 0 ? 0 : bx0; bx <= bx1 && bx < ntx; ++bx) {
           const int x0 = L + bx * TX, z0 = L + bz * TZ;
           if (v.i >= x0 - HV && v.i < x0 + TX + HV && v.j >= z0 - HV && v.j < z0 + TZ + HV)
-            per[bz * ntx + bx].push_back(make_int4(v.i, v.j, q, kind));
+            all.emplace_back(bz * ntx + bx, make_int4(v.i, v.j, q, kind));
         }
     }
     for (int r = 0; r < s->nrec; ++r) {
       const vi_receiver &v = s->rec_host[r];
-      per[own_tile(v.i, v.j)].push_back(make_int4(v.i, v.j, r, TL_RECEIVER));
+      all.emplace_back(own_tile(v.i, v.j), make_int4(v.i, v.j, r, TL_RECEIVER));
     }
   }
-  off.assign(ntiles + 1, 0);
-  ent.clear();
-  for (int t = 0; t < ntiles; ++t) {
-    // by kind (force, explosive, receiver), in their original order within
-    // a kind: a loop over one kind stops at the first entry of the next
-    std::stable_sort(per[t].begin(), per[t].end(), [](const int4 &u, const int4 &v) { return u.w < v.w; });
-    off[t] = (int)ent.size();
-    ent.insert(ent.end(), per[t].begin(), per[t].end());
+  // by tile, then kind (force, explosive, receiver), in their original order
+  // within a kind: a loop over one kind stops at the first entry of the next.
+  // The entries are sorted, not the tiles: a call's cost is its entries'.
+  std::stable_sort(all.begin(), all.end(), [](const auto &u, const auto &v) {
+    return u.first != v.first ? u.first < v.first : u.second.w < v.second.w;
+  });
+  off.assign(ntiles + 1, (int)all.size());
+  ent.resize(all.size());
+  int t = 0;
+  for (size_t k = 0; k < all.size(); ++k) {
+    while (t <= all[k].first) off[t++] = (int)k;
+    ent[k] = all[k].second;
   }
-  off[ntiles] = (int)ent.size();
+}
+
+static bool same_bytes(const std::vector<char> &have, const void *p, size_t n) {
+  return have.size() == n && (n == 0 || std::memcmp(have.data(), p, n) == 0);
 }
 
 int stage_tile_lists(vi_plan *p, const std::vector<int> &off, const std::vector<int4> &ent,
                      cudaStream_t st, int **d_off, int4 **d_ent) {
   const size_t ent_off = (off.size() * sizeof(int) + 15) / 16 * 16;
   const size_t lbytes = ent_off + ent.size() * sizeof(int4) + 16;
-  int rc = ensure_buffer(p, &p->tile_lists, &p->tile_lists_bytes, lbytes);
-  if (rc) return rc;
+  // one block, offsets then entries
+  std::vector<char> now(ent_off + ent.size() * sizeof(int4), 0);
+  std::memcpy(now.data(), off.data(), off.size() * sizeof(int));
+  if (!ent.empty()) std::memcpy(now.data() + ent_off, ent.data(), ent.size() * sizeof(int4));
+  int rc = VI_OK;
+  if (!p->tile_lists || !same_bytes(p->tile_lists_host, now.data(), now.size())) {
+    p->tile_lists_host.clear();
+    if ((rc = ensure_buffer(p, &p->tile_lists, &p->tile_lists_bytes, lbytes))) return rc;
+    rc = cuda_check(cudaMemcpyAsync(p->tile_lists, now.data(), now.size(), cudaMemcpyHostToDevice, st),
+                    "copy tile lists");
+    // the host block may go once the pageable copy is done; other streams find
+    // the lists complete
+    if (!rc) rc = cuda_check(cudaStreamSynchronize(st), "stage tile lists");
+    if (rc) return rc;
+    p->tile_lists_host.swap(now);
+  }
   *d_off = (int *)p->tile_lists;
   *d_ent = (int4 *)((char *)p->tile_lists + ent_off);
-  rc = cuda_check(cudaMemcpyAsync(*d_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice, st),
-                  "copy tile offsets");
-  if (rc) return rc;
-  if (!ent.empty()) {
-    rc = cuda_check(cudaMemcpyAsync(*d_ent, ent.data(), ent.size() * sizeof(int4), cudaMemcpyHostToDevice, st),
-                    "copy tile entries");
-    if (rc) return rc;
-  }
-  // the host vectors die at return: wait for the pageable copies
-  return cuda_check(cudaStreamSynchronize(st), "stage tile lists");
+  return VI_OK;
 }
 
 static bool aligned16(const void *ptr) { return ((uintptr_t)ptr & 15) == 0; }

@@ -55,7 +55,9 @@ int fused_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps
 // recomputed-velocity halo is HV cells (0 for the split kernels).
 void build_tile_lists(int nx, int nz, int TX, int TZ, int HV, const vi_shot *s,
                       std::vector<int> &off, std::vector<int4> &ent, int &ntx, int &ntz);
-// Copies the lists into the plan's device buffer (synchronizes `st`).
+// Copies the lists into the plan's device buffer (and synchronizes `st`), unless
+// it holds the same lists already: a time loop that comes back with the same
+// sources and receivers then queues its kernels behind the last call's.
 int stage_tile_lists(vi_plan *p, const std::vector<int> &off, const std::vector<int4> &ent,
                      cudaStream_t st, int **d_off, int4 **d_ent);
 

@@ -34,6 +34,8 @@ struct vi_plan {
   void *shadow = nullptr;
   size_t shadow_bytes = 0;
   unsigned shadow_pass = 1;
+  int res_geom[6] = {0, 0, 0, 0, 0, 0}, res_fits = -1;  // its tiling, once looked for
+  size_t res_smem = 0;
   // split step on grids whose rows need padding: state, medium, TTI's
   // second memory-variable set (grown on demand)
   void *pad = nullptr;
@@ -49,6 +51,8 @@ struct vi_plan {
   // fused path: per-tile source / receiver lists (device, grown on demand)
   void *tile_lists = nullptr;
   size_t tile_lists_bytes = 0;
+  // what the device lists hold (empty: nothing staged)
+  std::vector<char> tile_lists_host, src_host, amp_host, rec_host;
   // wavefront step: ticket, abort flag and per-band completion counters;
   // sweep depth (steps) and band lag, 0 = the built-in defaults
   void *wave_ctl = nullptr;

@@ -601,13 +601,29 @@ static bool res_geometry(const vi_config &c, int nsm, ResGeom &out) {
   return found;
 }
 
-bool resident_eligible_cfg(const vi_plan *p, int nsteps) {
+// the plan's tiling, looked for once
+template <typename T>
+static bool res_plan_geometry(vi_plan *p, ResGeom &g) {
+  if (p->res_fits < 0) {
+    p->res_fits = res_geometry<T>(p->cfg, p->nsm, g);
+    if (p->res_fits) {
+      const int v[6] = {g.txg, g.tz, g.px, g.pz, g.threads, g.width};
+      std::copy(v, v + 6, p->res_geom);
+      p->res_smem = g.smem;
+    }
+  }
+  const int *v = p->res_geom;
+  g = ResGeom{v[0], v[1], v[2], v[3], v[4], v[5], p->res_smem};
+  return p->res_fits == 1;
+}
+
+bool resident_eligible_cfg(vi_plan *p, int nsteps) {
   const vi_config &c = p->cfg;
   if (nsteps < kResidentMinSteps || p->no_resident || c.medium == VI_MEDIUM_TTI || c.precision == VI_F32C ||
       c.free_surface == kFsAfda || c.nx % 4 != 0)
     return false;
   ResGeom g;
-  if (!(c.precision == VI_F64 ? res_geometry<double>(c, p->nsm, g) : res_geometry<float>(c, p->nsm, g))) return false;
+  if (!(c.precision == VI_F64 ? res_plan_geometry<double>(p, g) : res_plan_geometry<float>(p, g))) return false;
   // with other plans' steps in flight only grids whose CTAs leave most of an SM
   // free: 8 streams of 128 x 128 VTI steps took 0.73 us per shot and step here
   // against 1.65 for the pair, of 512 x 256 4.7 against 2.7
@@ -642,7 +658,7 @@ template <typename T>
 int resident_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st) {
   const vi_config &c = p->cfg;
   ResGeom g;
-  if (!res_geometry<T>(c, p->nsm, g)) return set_error(VI_ERR_ARG, "resident step: the grid does not fit on the chip");
+  if (!res_plan_geometry<T>(p, g)) return set_error(VI_ERR_ARG, "resident step: the grid does not fit on the chip");
   int ntx, ntz;
   std::vector<int> off;
   std::vector<int4> ent;

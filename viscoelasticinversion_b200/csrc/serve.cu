@@ -226,6 +226,7 @@ int admit_impl(vi_server *s, Req &q) {
   int rc = cuda_check(cudaStreamCreateWithFlags(&q.st, cudaStreamNonBlocking), "serve: create stream");
   if (rc) return rc;
   if ((rc = take_plan(s, c, &q.plan))) return rc;
+  mark_call(q.plan, true);  // in flight as long as it is resident
   const int ns = 5 + 3 * c.nsls;
   const int nmed = 8;
   const size_t tr = 2 * (size_t)r.nrec * r.nt;
@@ -302,7 +303,10 @@ void release(vi_server *s, Req &q) {
   if (q.buf) cudaFreeAsync(q.buf, q.st);
   q.buf = nullptr;
   if (q.st) cudaStreamSynchronize(q.st);
-  if (q.plan) give_plan(s, q.plan);
+  if (q.plan) {
+    mark_call(q.plan, false);
+    give_plan(s, q.plan);
+  }
   q.plan = nullptr;
   if (q.st) cudaStreamDestroy(q.st);
   q.st = nullptr;
