@@ -235,7 +235,34 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
     }
     __syncthreads();
   }
+  // The value beside a group along the row comes from the next (or previous)
+  // lane in FP32: a 4-byte access per lane, 16 bytes apart, costs the L1 as much
+  // as a whole vector, and there are twelve a group (TTI pair at 2048x1024: 71.3 ->
+  // 69.5 us a step, 1024x512 20.6 -> 20.2).
+  // Lanes at the end of a tile row, or beside an idle lane, load it.  FP64 moves
+  // 8 bytes in two shuffles and gained nothing (55.9 vs 56.0 us at 1024x512), so
+  // it loads.
+  constexpr bool SHFL = sizeof(T) == 4;
+  constexpr int GPR = TX / 4 < 32 ? TX / 4 : 32;  // groups of a tile row within a warp
+  const unsigned live = __ballot_sync(0xffffffffu, act);
   if (!act) return;
+  const bool last = tid % GPR == GPR - 1 || gi0 + 4 >= xe, first = tid % GPR == 0;
+  auto next = [&](T v, auto load) -> T {
+    if constexpr (SHFL) {
+      const T n = __shfl_down_sync(live, v, 1);
+      return last ? load() : n;
+    } else {
+      return load();
+    }
+  };
+  auto prev = [&](T v, auto load) -> T {
+    if constexpr (SHFL) {
+      const T n = __shfl_up_sync(live, v, 1);
+      return first ? load() : n;
+    } else {
+      return load();
+    }
+  };
   // ---- stresses and memory variables of the own group
   const T dt = a.dt;
   const Q4<T> dt4 = splat4<T>(dt);
@@ -247,18 +274,25 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
   const Q4<T> c15a = ldg4(a.c15 + g), c15b = ldg4(a.c15 + g + ld);
   const Q4<T> c35a = ldg4(a.c35 + g), c35b = ldg4(a.c35 + g + ld);
   const Q4<T> c55a = ldg4(a.c55 + g), c55b = ldg4(a.c55 + g + ld);
-  const T c15a4 = __ldg(a.c15 + g + 4), c15b4 = __ldg(a.c15 + g + ld + 4);
-  const T c35a4 = __ldg(a.c35 + g + 4), c35b4 = __ldg(a.c35 + g + ld + 4);
-  const T c55a4 = __ldg(a.c55 + g + 4), c55b4 = __ldg(a.c55 + g + ld + 4);
+  const T c15a4 = next(c15a.v[0], [&] { return __ldg(a.c15 + g + 4); });
+  const T c15b4 = next(c15b.v[0], [&] { return __ldg(a.c15 + g + ld + 4); });
+  const T c35a4 = next(c35a.v[0], [&] { return __ldg(a.c35 + g + 4); });
+  const T c35b4 = next(c35b.v[0], [&] { return __ldg(a.c35 + g + ld + 4); });
+  const T c55a4 = next(c55a.v[0], [&] { return __ldg(a.c55 + g + 4); });
+  const T c55b4 = next(c55b.v[0], [&] { return __ldg(a.c55 + g + ld + 4); });
   const int e = (r + 1) * EW + lx + 4;
   const Q4<T> exx = lds4(s_exx + e), ezz = lds4(s_ezz + e), exz = lds4(s_exz + e);
   // e_xz at the integer node: mean of (i-1/2, j-1/2) .. (i+1/2, j+1/2)
   const Q4<T> xzm = lds4(s_exz + e - EW);
   const Q4<T> ebxz = mul4(splat4<T>(T(0.25)),
-                          add4(add4(add4(exz, prev4(exz, s_exz[e - 1])), xzm), prev4(xzm, s_exz[e - EW - 1])));
+                          add4(add4(add4(exz, prev4(exz, prev(exz.v[3], [&] { return s_exz[e - 1]; }))), xzm),
+                               prev4(xzm, prev(xzm.v[3], [&] { return s_exz[e - EW - 1]; }))));
   // e_xx, e_zz at the half node: mean of (i, j) .. (i+1, j+1)
-  const Q4<T> ebxx = mean4_fwd(exx, s_exx[e + 4], lds4(s_exx + e + EW), s_exx[e + EW + 4]);
-  const Q4<T> ebzz = mean4_fwd(ezz, s_ezz[e + 4], lds4(s_ezz + e + EW), s_ezz[e + EW + 4]);
+  const Q4<T> exxb = lds4(s_exx + e + EW), ezzb = lds4(s_ezz + e + EW);
+  const Q4<T> ebxx = mean4_fwd(exx, next(exx.v[0], [&] { return s_exx[e + 4]; }), exxb,
+                               next(exxb.v[0], [&] { return s_exx[e + EW + 4]; }));
+  const Q4<T> ebzz = mean4_fwd(ezz, next(ezz.v[0], [&] { return s_ezz[e + 4]; }), ezzb,
+                               next(ezzb.v[0], [&] { return s_ezz[e + EW + 4]; }));
   const Q4<T> C15h = mean4_fwd(c15a, c15a4, c15b, c15b4);
   const Q4<T> C35h = mean4_fwd(c35a, c35a4, c35b, c35b4);
   const Q4<T> C55h = mean4_fwd(c55a, c55a4, c55b, c55b4);
