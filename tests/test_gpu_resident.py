@@ -59,6 +59,28 @@ def test_resident_form_runs_and_reports_nonfinite():
     plan.close()
 
 
+def test_plans_taking_turns_on_a_stream_stay_resident():
+    # blocks of more than 128 threads: resident unless other streams' steps are in flight
+    from torch.profiler import ProfilerActivity, profile
+
+    w = media.layered(nx=256, nz=256, nt=90, kind="iso", seed=5, pml=12, nrec=8)
+    plans = [StepPlan.for_workload(w, "f64") for _ in range(3)]
+    med = plans[0].medium_to_device(w.medium)
+    states = [p.zeros_state() for p in plans]
+    for p, s in zip(plans, states):
+        p.step(med, s, nsteps=20)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        for _ in range(3):
+            for p, s in zip(plans, states):
+                p.step(med, s, nsteps=20)
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events()]
+    assert sum("k_resident" in n for n in names) >= 9 and not any("k_split" in n for n in names)
+    for p in plans:
+        p.status()
+        p.close()
+
+
 def test_resident_steps_on_several_streams():
     """Plans stepped from several streams at once give their own results."""
     works = [media.layered(nx=nx, nz=nz, nt=64, kind="vti", seed=nx, pml=10, nrec=6)

@@ -29,6 +29,7 @@ struct vi_plan {
   // whether work of this plan may still run: recorded after each longer step
   // call, in_call during a gradient (both under capi.cu's list of plans)
   cudaEvent_t done = nullptr;
+  cudaStream_t done_stream = nullptr;
   bool done_pending = false, in_call = false;
   // resident steps: the tiles' edges beside the pass that wrote them
   void *shadow = nullptr;
@@ -78,9 +79,9 @@ struct vi_plan {
 namespace vb {
 int set_error(int code, const std::string &msg);
 // Whether another plan of this process has steps or a gradient in flight on the
-// device (the resident step, which takes whole SMs, then leaves it to kernels
-// that run side by side); marks for this plan.
-bool others_in_flight(const vi_plan *p);
+// device that are not queued on st itself (the resident step, which takes whole
+// SMs, then leaves it to kernels that run side by side); marks for this plan.
+bool others_in_flight(const vi_plan *p, cudaStream_t st);
 void mark_steps(vi_plan *p, cudaStream_t st);
 void mark_call(vi_plan *p, bool running);
 int cuda_check(cudaError_t e, const char *what);

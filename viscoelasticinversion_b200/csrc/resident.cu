@@ -617,7 +617,7 @@ static bool res_plan_geometry(vi_plan *p, ResGeom &g) {
   return p->res_fits == 1;
 }
 
-bool resident_eligible_cfg(vi_plan *p, int nsteps) {
+bool resident_eligible_cfg(vi_plan *p, int nsteps, cudaStream_t st) {
   const vi_config &c = p->cfg;
   if (nsteps < kResidentMinSteps || p->no_resident || c.medium == VI_MEDIUM_TTI || c.precision == VI_F32C ||
       c.free_surface == kFsAfda || c.nx % 4 != 0)
@@ -627,7 +627,7 @@ bool resident_eligible_cfg(vi_plan *p, int nsteps) {
   // with other plans' steps in flight only grids whose CTAs leave most of an SM
   // free: 8 streams of 128 x 128 VTI steps took 0.73 us per shot and step here
   // against 1.65 for the pair, of 512 x 256 4.7 against 2.7
-  return g.threads <= 128 || !others_in_flight(p);
+  return g.threads <= 128 || !others_in_flight(p, st);
 }
 
 template <typename T, int KIND, int NSLS, int W>

@@ -157,7 +157,7 @@ int wave_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps,
 // 512 174 against 202; about 40 us of loading, launching and storing are won
 // back in some 5 steps).
 constexpr int kResidentMinSteps = 16;
-bool resident_eligible_cfg(vi_plan *p, int nsteps);
+bool resident_eligible_cfg(vi_plan *p, int nsteps, cudaStream_t st);
 template <typename T>
 int resident_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps, cudaStream_t st);
 
