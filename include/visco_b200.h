@@ -170,7 +170,8 @@ int vi_plan_workspace_bytes(const vi_plan *plan, int64_t *bytes);
  * reaches the caller. */
 int vi_plan_status(vi_plan *plan, void *stream);
 /* Which kernel the last vi_step ran: 1 plain, 2 fused, 3 fused TMA-staged,
- * 4 fused TMA-staged single-stage, 5 split velocity/stress pair, 6 split
+ * 4 fused TMA-staged single-stage, 5 split velocity/stress pair (its
+ * resident and padded forms included), 6 split
  * pair, persistent and TMA-pipelined, 7 streaming, 8 split pair with the
  * direct-load velocity pass. */
 int vi_plan_last_kernel(const vi_plan *plan, int32_t *kernel);
@@ -186,7 +187,11 @@ int vi_plan_last_kernel(const vi_plan *plan, int32_t *kernel);
  * (free-surface-kernels.jl:16-213) and the CPML/ψ recursion
  * (sciml_solver/CPML.jl:291-328).  `shot` may be NULL (no sources or
  * receivers).  kernel_variant: 0 = default (with nx % 4 == 0 and 16-byte
- * aligned planes the split pair, else the fused kernel), 1 = plain
+ * aligned planes the split pair, for small ISO/VTI grids and enough steps
+ * as one resident kernel per call; other rows and planes of 2048 cells or
+ * more on padded copies that the plan allocates, copied in and out every
+ * call; the fused kernel for smaller ones and when there is no memory for
+ * the copies), 1 = plain
  * multi-kernel path (in place), 2 = fused kernel without TMA, 3 = TMA-staged
  * fused kernel (persistent, two stages when they fit), 4 = TMA-staged fused
  * kernel with one stage, 5 = split velocity/stress kernel pair (one tile
@@ -299,7 +304,9 @@ int vi_batch_status(vi_batch *batch, void *stream, int32_t *kernel_form);
  * state of the forward sweep in HBM when they fit in 60 % of the device's
  * memory and in what is free (nothing recomputed; 88 GB for a 1024 x 512,
  * 3000-step VTI FP32 shot), else checkpoints every ceil(sqrt(nt)) steps.
- * The result is bitwise the same for every interval.  accumulate != 0 adds into grad_dev
+ * The result is bitwise the same for every interval.  State, medium copies
+ * of rows that are no multiple of 16 bytes, and adjoint planes are laid out
+ * with padded rows in the workspace.  accumulate != 0 adds into grad_dev
  * (shots summed), else grad_dev is overwritten.  *misfit_host = J (FP64).
  * The shot's traces_dev, if given with traces_nt >= nt, receives d.
  * Synchronous on `stream`. */

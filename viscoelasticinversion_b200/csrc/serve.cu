@@ -119,7 +119,7 @@ double remaining_work(const Req &q) {
 }
 
 // Device bytes a request holds while resident (plan workspace included,
-// rounded up): medium, state, the fused path's second state copy, CPML
+// rounded up): medium, state, the second state or padded copy, CPML
 // strips, wavelets and traces; for a gradient the checkpoints and segment
 // slots, the adjoint state and scratch, observed traces and FP64 planes.
 int64_t footprint(const vi_request &r) {
