@@ -63,16 +63,28 @@ bool others_in_flight(const vi_plan *p, cudaStream_t st) {
     if (q == p || q->device != p->device) continue;
     if (q->in_call) return true;
     if (!q->done_pending || (q->done_stream == st && st != cudaStreamPerThread)) continue;
-    if (cudaEventQuery(q->done) == cudaErrorNotReady) {
-      cudaGetLastError();
-      return true;
-    }
+    const cudaError_t e = cudaEventQuery(q->done);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e == cudaErrorNotReady) return true;
     q->done_pending = false;
   }
   return false;
 }
 
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+  cudaGetLastError();  // the legacy stream beside another stream's capture
+  return true;
+}
+int refuse_capture(cudaStream_t st) {
+  return capturing(st) ? set_error(VI_ERR_CUDA, "a step that stages lists cannot be captured: its arguments hold the "
+                                                "plan's state of this call")
+                       : VI_OK;
+}
+
 void mark_steps(vi_plan *p, cudaStream_t st) {
+  if (capturing(st)) return;  // an event of the graph says nothing about its runs
   std::lock_guard<std::mutex> lk(g_plans_mu);
   if (!p->done && cudaEventCreateWithFlags(&p->done, cudaEventDisableTiming) != cudaSuccess) {
     cudaGetLastError();
@@ -338,6 +350,8 @@ template <typename T>
 int stage_shot(vi_plan *p, const vi_shot *s, cudaStream_t st) {
   if (!s) return VI_OK;
   if (s->nsrc < 0 || s->nrec < 0) return set_error(VI_ERR_ARG, "negative source/receiver count");
+  if (s->nsrc > 0 || s->nrec > 0)
+    if (const int rc = refuse_capture(st)) return rc;
   if (s->nsrc > 0) {
     if (!s->src_host || !s->wavelet_dev || s->wavelet_nt < 0)
       return set_error(VI_ERR_ARG, "sources need src_host and wavelet_dev");

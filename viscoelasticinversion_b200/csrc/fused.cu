@@ -432,7 +432,8 @@ int stage_tile_lists(vi_plan *p, const std::vector<int> &off, const std::vector<
   std::vector<char> now(ent_off + ent.size() * sizeof(int4), 0);
   std::memcpy(now.data(), off.data(), off.size() * sizeof(int));
   if (!ent.empty()) std::memcpy(now.data() + ent_off, ent.data(), ent.size() * sizeof(int4));
-  int rc = VI_OK;
+  int rc = refuse_capture(st);
+  if (rc) return rc;
   if (!p->tile_lists || !same_bytes(p->tile_lists_host, now.data(), now.size())) {
     p->tile_lists_host.clear();
     if ((rc = ensure_buffer(p, &p->tile_lists, &p->tile_lists_bytes, lbytes))) return rc;

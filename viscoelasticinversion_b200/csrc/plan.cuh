@@ -83,6 +83,12 @@ int set_error(int code, const std::string &msg);
 // SMs, then leaves it to kernels that run side by side); marks for this plan.
 bool others_in_flight(const vi_plan *p, cudaStream_t st);
 void mark_steps(vi_plan *p, cudaStream_t st);
+// Whether st records a graph; an error when it does.  The step's arguments hold
+// what changes from call to call (the resident form's pass numbers, the buffer
+// of TTI's memory variables that is current), so a graph of it must not be
+// replayed; list staging refuses it whether or not it has something to copy.
+bool capturing(cudaStream_t st);
+int refuse_capture(cudaStream_t st);
 void mark_call(vi_plan *p, bool running);
 int cuda_check(cudaError_t e, const char *what);
 // Grow-only device buffer.
