@@ -538,6 +538,14 @@ __device__ __forceinline__ void zero_outside(Pk<T> &q, int n) {
   for (int k = 0; k < VecW<T>::V; ++k)
     if (k >= n) q.v[k] = T(0);
 }
+// The medium of lanes past the update region is the caller's and may be anything
+// (0 x inf is NaN): their moduli and tau count as 0, what divides as 1.
+template <typename T>
+__device__ __forceinline__ void set_outside(Pk<T> &q, int n, T v) {
+#pragma unroll
+  for (int k = 0; k < VecW<T>::V; ++k)
+    if (k >= n) q.v[k] = v;
+}
 // u[k + 1] of the group, u[V] from `next`
 template <typename T>
 __device__ __forceinline__ T right_of(const Pk<T> &u, int k, T next) {
@@ -705,8 +713,6 @@ __global__ void __launch_bounds__(AdjGeom<T>::NT, N <= 3 ? 2 : 1)
   stv(sb + 2 * np + c, bxz);
   Pk<T> rt[3], e[3];
   adj_rates(A, x0, s, t, box(SM::VX) + ow + 3 * G::WX, box(SM::VZ) + ow + 4 * G::WX, rt);
-#pragma unroll
-  for (int k = 0; k < 3; ++k) e[k] = N > 0 ? pfma(tau, padd(rt[k], S[k]), rt[k]) : rt[k];
   const T *cc = box(SM::CC) + oc;
   const Pk<T> c55 = ldv(cc), c55d = ldv(cc + G::WC);
   Pk<T> C55h;
@@ -714,6 +720,15 @@ __global__ void __launch_bounds__(AdjGeom<T>::NT, N <= 3 ? 2 : 1)
   for (int k = 0; k < V; ++k)
     C55h.v[k] = T(0.25) * (c55.v[k] + right_of(c55, k, cc[V]) + c55d.v[k] + right_of(c55d, k, cc[G::WC + V]));
   if (KIND == VI_MEDIUM_ISO) C11 = C33 = pfma(splat<T>(T(2)), c55, C13);
+  if (const int n = A.nx - L - t.gi0; n < V) {
+    zero_outside(tau, n);
+    zero_outside(C11, n);
+    zero_outside(C13, n);
+    set_outside(C33, n, T(1));
+    zero_outside(C55h, n);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) e[k] = N > 0 ? pfma(tau, padd(rt[k], S[k]), rt[k]) : rt[k];
   // accumulators: plane 0 TAU, 1 Q55, 2 C11 (ISO: C11 and C33), 3 C13, 4 C33
   const double *ai = reinterpret_cast<const double *>(smem + SM::ACC) + oz;
   double *ao = acc + c;
@@ -845,6 +860,10 @@ __global__ void __launch_bounds__(AdjGeom<T>::NT, 5)
     bx.v[k] = T(2) / (r0.v[k] + right_of(r0, k, rr));
     bz.v[k] = T(2) / (r0.v[k] + r1.v[k]);
   }
+  if (t.gi0 + V > A.nx - L) {
+    zero_outside(bx, A.nx - L - t.gi0);
+    zero_outside(bz, A.nx - L - t.gi0);
+  }
   for (int e = e0; e < e1; ++e) {  // force sources: their buoyancy factor depends on rho too
     const int4 en = x.tile_ent[e];
     if (en.w > TL_FORCE_Z) break;
@@ -965,6 +984,16 @@ __device__ __forceinline__ Row3<T> ldrow3(const T *u) {
   for (int k = 0; k < V; ++k) r.w[1 + k] = t.v[k];
   return r;
 }
+// the same of a modulus, 0 before the update region (no updated cell reads
+// it there; the sigma adjoint it meets is 0)
+template <typename T>
+__device__ __forceinline__ Row3<T> ldrow3_med(const T *u, const AdjTile &t, int j) {
+  Row3<T> r{};
+  if (j < L) return r;
+  r = ldrow3(u);
+  if (t.gi0 == L) r.w[0] = T(0);
+  return r;
+}
 // mean of the four cells (i, j), (i+1, j), (i, j+1), (i+1, j+1), cell o - 1 of
 // the group (o = 0: the cell before it)
 template <typename T>
@@ -996,6 +1025,12 @@ __global__ void __launch_bounds__(AdjGeom<T>::NT, 3)
     C13 = ldn(A.c13 + c);
     C33 = ldn(A.c33 + c);
     if (N > 0) tau = ldn(A.tau + c);
+    if (const int n = A.nx - L - t.gi0; n < V) {
+      zero_outside(tau, n);
+      zero_outside(C11, n);
+      zero_outside(C13, n);
+      set_outside(C33, n, T(1));
+    }
 #pragma unroll
     for (int q = 0; q < 3 * N; ++q) mb[q] = ldcgv(mbar + q * np + c);
   }
@@ -1050,7 +1085,7 @@ __global__ void __launch_bounds__(AdjGeom<T>::NT, 3)
     }
     {
       const T *a = box(SM::C15) + o;
-      const Row3<T> a0 = ldrow3(a), ap = ldrow3(a + W), am = ldrow3(a - W);
+      const Row3<T> a0 = ldrow3_med(a, t, t.j), ap = ldrow3_med(a + W, t, t.j + 1), am = ldrow3_med(a - W, t, t.j - 1);
       const Row3<T> sx0 = ldrow3(b0), sxp = ldrow3(b0 + W);
 #pragma unroll
       for (int k = 0; k < V; ++k) {
@@ -1063,7 +1098,7 @@ __global__ void __launch_bounds__(AdjGeom<T>::NT, 3)
     }
     {
       const T *a = box(SM::C35) + o;
-      const Row3<T> a0 = ldrow3(a), ap = ldrow3(a + W), am = ldrow3(a - W);
+      const Row3<T> a0 = ldrow3_med(a, t, t.j), ap = ldrow3_med(a + W, t, t.j + 1), am = ldrow3_med(a - W, t, t.j - 1);
       const Row3<T> sz0 = ldrow3(b0 + RP), szp = ldrow3(b0 + RP + W);
 #pragma unroll
       for (int k = 0; k < V; ++k) {
@@ -1126,6 +1161,7 @@ __global__ void __launch_bounds__(AdjGeom<T>::NT, 3)
       wz.v[k] = c35own.v[k] / C33.v[k] * zb.v[k];
       eb[0].v[k] -= C13.v[k] / C33.v[k] * zb.v[k];
     }
+    if (t.gi0 + V > A.nx - L) zero_outside(wz, A.nx - L - t.gi0);
 #pragma unroll
     for (int k = 0; k < V; ++k) eb[2].v[k] -= T(0.25) * (wz.v[k] + right_of(wz, k, wr * zr));
     eb[1] = splat<T>(T(0));
