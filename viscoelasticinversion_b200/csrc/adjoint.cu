@@ -557,22 +557,28 @@ __device__ __forceinline__ T right_of(const Pk<T> &u, int k, T next) {
 // velocity stage after it, with the images transposed: row L + k also takes
 // what -D^T dbar leaves on the ghost rows L - k (szz) and L - 1 - k (sxz),
 // whose only terms are those dbar rows at or below the surface (within four
-// rows of row L + k, so inside its boxes).  sb, d0 .. d3: the group's place in the boxes.
+// rows of row L + k, so inside its boxes).  The image terms join the derivative
+// first, so the running sigma adjoint is rounded once.  sb, d0 .. d3: the group's
+// place in the boxes.
 template <typename T>
 __device__ __forceinline__ void adj_sigma(const AdjArgs<T> &A, const AdjTile &t, const T *sb, const T *d0, const T *d1,
                                           const T *d2, const T *d3, Pk<T> &bxx, Pk<T> &bzz, Pk<T> &bxz) {
   using G = AdjGeom<T>;
   bxx = psub(ldv(sb), dxm(ldwin(d0), A.Dx));
-  bzz = psub(ldv(sb + G::TX * G::TZ), dzm(d3, G::TX, A.Dz));
-  bxz = psub(ldv(sb + 2 * G::TX * G::TZ), padd(dzp(d1, G::TX, A.Dz), dxp(ldwin(d2), A.Dx)));
+  Pk<T> tzz = dzm(d3, G::TX, A.Dz), txz = padd(dzp(d1, G::TX, A.Dz), dxp(ldwin(d2), A.Dx));
   if (A.fs && t.j < 2 * L) {
     const int k = t.j - L;
+    Pk<T> izz = splat<T>(T(0)), ixz = izz;
     for (int q = k; q < 4; ++q) {  // grid row L - k + q: 2 k - q rows up from row L + k
       const T d = A.Dz[q];
-      bxz = pfma(splat<T>(d), ldv(d1 + (q - 2 * k) * G::TX), bxz);
-      if (k >= 1) bzz = pfma(splat<T>(d), ldv(d3 + (q - 2 * k) * G::TX), bzz);
+      ixz = pfma(splat<T>(d), ldv(d1 + (q - 2 * k) * G::TX), ixz);
+      if (k >= 1) izz = pfma(splat<T>(d), ldv(d3 + (q - 2 * k) * G::TX), izz);
     }
+    tzz = psub(tzz, izz);
+    txz = psub(txz, ixz);
   }
+  bzz = psub(ldv(sb + G::TX * G::TZ), tzz);
+  bxz = psub(ldv(sb + 2 * G::TX * G::TZ), txz);
   if (t.gi0 + G::V > A.nx - L) {
     zero_outside(bxx, A.nx - L - t.gi0);
     zero_outside(bzz, A.nx - L - t.gi0);
@@ -580,6 +586,15 @@ __device__ __forceinline__ void adj_sigma(const AdjArgs<T> &A, const AdjTile &t,
   }
 }
 
+// Effective rates of the forward step, rounded as its kernels round them: with
+// 1 + tau as one FP32 number.  The transpose uses the same number (adj_memory);
+// with tau applied by itself it transposed a slightly other step, and the FP32
+// gradient was 10 to 17 % further from the 64-bit one in rho, 4 to 12 % in the
+// other planes (256 x 160, 48 shots; with it, as far as unfused transposes).
+template <typename T>
+__device__ __forceinline__ Pk<T> effective_rate(const Pk<T> &tau, const Pk<T> &rt, const Pk<T> &S) {
+  return pfma(padd(tau, splat<T>(T(1))), rt, pmul(tau, S));
+}
 // Forward strain rates of the step from the new velocities (vx, vz: the
 // group's place in the boxes) and the CPML memory before it (x0): xx, zz, xz.
 template <typename T>
@@ -610,7 +625,7 @@ __device__ __forceinline__ void adj_memory(const AdjArgs<T> &A, F mb, T *mp, T *
   const long long np = A.np;
   Pk<T> rtb[3];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) rtb[k] = N > 0 ? pfma(tau, eb[k], eb[k]) : eb[k];
+  for (int k = 0; k < 3; ++k) rtb[k] = N > 0 ? pmul(padd(tau, splat<T>(T(1))), eb[k]) : eb[k];
 #pragma unroll
   for (int n = 0; n < N; ++n) {
     const T e1 = A.dt * A.a1[n], e2 = T(1) + A.dt * A.a2[n];
@@ -622,7 +637,7 @@ __device__ __forceinline__ void adj_memory(const AdjArgs<T> &A, F mb, T *mp, T *
       } else {
         const Pk<T> m = mb(k * N + n);
         rtb[k] = pfma(splat<T>(e1), m, rtb[k]);
-        stvp(q, pfma(tau, eb[k], pscale(e2, m)), l2_stream());
+        stvp(q, pfma(splat<T>(e2), m, pmul(tau, eb[k])), l2_stream());  // one rounding at the size of m
       }
     }
   }
@@ -728,7 +743,7 @@ __global__ void __launch_bounds__(AdjGeom<T>::NT, N <= 3 ? 2 : 1)
     zero_outside(C55h, n);
   }
 #pragma unroll
-  for (int k = 0; k < 3; ++k) e[k] = N > 0 ? pfma(tau, padd(rt[k], S[k]), rt[k]) : rt[k];
+  for (int k = 0; k < 3; ++k) e[k] = N > 0 ? effective_rate(tau, rt[k], S[k]) : rt[k];
   // accumulators: plane 0 TAU, 1 Q55, 2 C11 (ISO: C11 and C33), 3 C13, 4 C33
   const double *ai = reinterpret_cast<const double *>(smem + SM::ACC) + oz;
   double *ao = acc + c;
@@ -961,7 +976,7 @@ __global__ void __launch_bounds__(AdjGeom<T>::NT, 4)
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const Pk<T> rs = padd(rt[k], S[k]);
-    Pk<T> e = N > 0 ? pfma(tau, rs, rt[k]) : rt[k];
+    Pk<T> e = N > 0 ? effective_rate(tau, rt[k], S[k]) : rt[k];
     if (t.gi0 + G::V > A.nx - L) zero_outside(e, A.nx - L - t.gi0);
     stv(fe + k * np + c, e);
     stv(fe + (3 + k) * np + c, rs);
