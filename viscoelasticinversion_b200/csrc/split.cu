@@ -96,11 +96,11 @@ __global__ void __launch_bounds__(SplitGeom<T>::NT, (sizeof(T) == 4 ? 1024 : 512
   split_vel_sample<T>(b.args[2 * shot + (it & 1)], x, tile);
 }
 
-template <typename T, int KIND, int NSLS, bool OOP, bool HINT, bool COMP, bool AFDA>
+template <typename T, int KIND, int NSLS, bool OOP, bool HINT, bool COMP, bool AFDA, bool RAG>
 __global__ void __launch_bounds__(SplitStressGeom<T>::NT, (sizeof(T) == 4 ? 512 : 256) / SplitStressGeom<T>::NT)
     k_split_stress(const __grid_constant__ StepArgs<T> a, const __grid_constant__ FusedExtras<T> x,
                    const __grid_constant__ SplitMaps maps) {
-  split_stress_tile<T, KIND, NSLS, OOP, HINT, COMP, AFDA, SplitStressGeom<T>, true>(a, x, maps, blockIdx.x);
+  split_stress_tile<T, KIND, NSLS, OOP, HINT, COMP, AFDA, SplitStressGeom<T>, true, RAG>(a, x, maps, blockIdx.x);
 }
 
 template <typename T, int KIND, int NSLS, bool COMP, bool AFDA>
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(SplitStressGeomBatch<T>::NT, (sizeof(T) == 4 ?
 }
 
 // ------------------------------------------------------------------- host
-template <typename T, int KIND, int NSLS, bool OOP, bool HINT, bool COMP = false, bool AFDA = false>
+template <typename T, int KIND, int NSLS, bool OOP, bool HINT, bool COMP = false, bool AFDA = false, bool RAG = false>
 static int launch_stress_k(const StepArgs<T> &a, const FusedExtras<T> &x, const SplitMaps &m,
                            int ntiles, cudaStream_t st, bool pdl) {
   using SG = SplitStressGeom<T>;
@@ -130,12 +130,12 @@ static int launch_stress_k(const StepArgs<T> &a, const FusedExtras<T> &x, const 
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(attr_set & (1ULL << dev))) {
-    cudaError_t e = cudaFuncSetAttribute(k_split_stress<T, KIND, NSLS, OOP, HINT, COMP, AFDA>,
+    cudaError_t e = cudaFuncSetAttribute(k_split_stress<T, KIND, NSLS, OOP, HINT, COMP, AFDA, RAG>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, SG::SMEM);
     if (e != cudaSuccess) return cuda_check(e, "split stress smem attribute");
     attr_set |= 1ULL << dev;
   }
-  return cuda_check(launch_pdl(k_split_stress<T, KIND, NSLS, OOP, HINT, COMP, AFDA>, dim3(ntiles), dim3(SG::NT),
+  return cuda_check(launch_pdl(k_split_stress<T, KIND, NSLS, OOP, HINT, COMP, AFDA, RAG>, dim3(ntiles), dim3(SG::NT),
                                (size_t)SG::SMEM, st, pdl, a, x, m),
                     "split stress launch");
 }
@@ -146,7 +146,13 @@ template <typename T, int KIND, int NSLS>
 static int launch_stress(const StepArgs<T> &a, const FusedExtras<T> &x, const SplitMaps &m,
                          int ntiles, cudaStream_t st, bool pdl) {
   // the out-of-place form (the gradient's recompute) always hints
-  if (a.sxx_o) return launch_stress_k<T, KIND, NSLS, true, true>(a, x, m, ntiles, st, pdl);
+  const bool rag = a.nx % 4 != 0;  // planes padded by the plan: plain FP32 or FP64, imaging surface or none
+  if (a.sxx_o)
+    return rag ? launch_stress_k<T, KIND, NSLS, true, true, false, false, true>(a, x, m, ntiles, st, pdl)
+               : launch_stress_k<T, KIND, NSLS, true, true>(a, x, m, ntiles, st, pdl);
+  if (rag)
+    return x.l2hint ? launch_stress_k<T, KIND, NSLS, false, true, false, false, true>(a, x, m, ntiles, st, pdl)
+                    : launch_stress_k<T, KIND, NSLS, false, false, false, false, true>(a, x, m, ntiles, st, pdl);
   if constexpr (sizeof(T) == 4) {
     if (a.slo) {
       if (x.fs == kFsAfda)

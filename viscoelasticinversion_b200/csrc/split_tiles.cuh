@@ -29,7 +29,12 @@ namespace vb {
 // OOP: the new velocities go to a.vx_o / a.vz_o (a step from one state
 // buffer into another); else in place.  RAG: nx % 4 != 0, the last group of
 // a row reaches past the update region (an instantiation of its own: keeping
-// the old velocities for it cost the others 0.7 % of a TTI step).
+// the old velocities for it cost the others 0.7 % of a TTI step).  The RAG
+// kernels take FP32 z derivatives as differences of rows, as the fused and the
+// plain kernels do: tap by tap, v and sigma after 60 FP32 steps of 403 x 297 were 1.2
+// and 1.5 % further from the FP64 ones (1403 x 597 VTI, 60 steps: 1473 us tap by
+// tap, 1442 by differences; the FP64 gradient of 301 x 203 ran 1.4 % longer with
+// them, for a difference in the sixteenth digit).
 template <typename T, bool PP, bool OOP, bool HINT, bool RAG>
 __device__ __forceinline__ void split_vel_finish(const StepArgs<T> &a, const FusedExtras<T> &x, int tile,
                                                  int gi0, int gj, long long g, const Q4<T> &vxi,
@@ -142,6 +147,10 @@ __device__ __forceinline__ void split_vel_tile(const StepArgs<T> &a, const Fused
       zzz = fma4(splat4<T>(cq), v, zzz);
     }
   }
+  if constexpr (RAG && sizeof(T) == 4) {
+    zxz = dzm_rows4(a.Dz, [&](int q) { return q == 0 ? win4(hxz, 4) : ldg4(a.sxz + g + (long long)q * ld); });
+    zzz = dzp_rows4(a.Dz, [&](int q) { return ldg4(a.szz + g + (long long)q * ld); });
+  }
   if (AFDA && gj < L + 4) {  // one-sided z derivatives below the H-AFDA surface
     const int qs = gj - L;
     zxz = afda4<0>(a, qs, [&](int m) { return ldg4(a.sxz + (long long)(L + m) * ld + gi0); });
@@ -245,6 +254,10 @@ __device__ __forceinline__ void split_vel_tma_tile(const StepArgs<T> &a, const F
       zzz = fma4(splat4<T>(cq), v, zzz);
     }
   }
+  if constexpr (RAG && sizeof(T) == 4) {
+    zxz = dzm_rows4(a.Dz, [&](int q) { return q == 0 ? win4(hxz, 4) : lds4(s_sxz + (r + 4 + q) * WX + lx + 4); });
+    zzz = dzp_rows4(a.Dz, [&](int q) { return lds4(s_szz + (r + 4 + q) * WZ + lx); });
+  }
   static_assert(G::TZ >= 4, "the H-AFDA rows below the surface lie in the first tile row");
   if (AFDA && gj < L + 4) {  // one-sided z derivatives below the H-AFDA surface (z0 == L)
     const int qs = gj - L;
@@ -263,9 +276,10 @@ __device__ __forceinline__ void split_vel_tma_tile(const StepArgs<T> &a, const F
 // kernel's PDL wait comes after the loads of sigma, M and the medium (state
 // the previous stress pass wrote: complete before the velocity pass that
 // precedes this grid released it), and the next grid is released at once;
-// else the wait comes first and the next grid is released at exit.
+// else the wait comes first and the next grid is released at exit.  RAG: nx % 4
+// != 0 (FP32 z derivatives as split_vel_finish says).
 template <typename T, int KIND, int NSLS, bool OOP, bool HINT, bool COMP = false, bool AFDA = false,
-          typename G = SplitStressGeom<T>, bool EARLY = false>
+          typename G = SplitStressGeom<T>, bool EARLY = false, bool RAG = false>
 __device__ __forceinline__ void split_stress_tile(const StepArgs<T> &a, const FusedExtras<T> &x,
                                                   const SplitMaps &maps, int tile) {
   static_assert(!COMP || (sizeof(T) == 4 && !OOP), "compensated stress: FP32, in place");
@@ -354,6 +368,10 @@ __device__ __forceinline__ void split_stress_tile(const StepArgs<T> &a, const Fu
       const Q4<T> v = q == 0 ? win4(hvx, 4) : lds4(s_vx + vb + q * SW + 4);
       zvx = fma4(splat4<T>(cq), v, zvx);
     }
+  }
+  if constexpr (RAG && sizeof(T) == 4) {
+    zvz = dzm_rows4(a.Dz, [&](int q) { return q == 0 ? win4(hvz, 4) : lds4(s_vz + vb + q * SW + 4); });
+    zvx = dzp_rows4(a.Dz, [&](int q) { return q == 0 ? win4(hvx, 4) : lds4(s_vx + vb + q * SW + 4); });
   }
   if (AFDA && gj < L + 4) {  // one-sided z derivatives below the H-AFDA surface (grid row L + m
     const int qs = gj - L;     // is box row L + m - (z0 - 4); on the surface row the tau_zz = 0

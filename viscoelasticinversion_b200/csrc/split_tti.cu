@@ -34,7 +34,8 @@ namespace vb {
 // AFDA: the grid has the H-AFDA surface, under which the z derivatives of
 // the four rows below it are one-sided (v box row of grid row L + m:
 // wb + (L + m - gj) * BW).
-template <typename T, int BW, bool AFDA>
+// RAG: FP32 z derivatives as differences of rows (split_vel_finish says why).
+template <typename T, int BW, bool AFDA, bool RAG>
 __device__ __forceinline__ void tti_rates4(const StepArgs<T> &a, const T *s_vx, const T *s_vz,
                                            int wb, int gi0, int gj, bool own, Q4<T> &rxx,
                                            Q4<T> &rzz, Q4<T> &rxz) {
@@ -54,6 +55,10 @@ __device__ __forceinline__ void tti_rates4(const StepArgs<T> &a, const T *s_vx, 
       const Q4<T> v = q == 0 ? win4(hvx, 4) : lds4(s_vx + wb + q * BW + 4);
       zvx = fma4(splat4<T>(cq), v, zvx);
     }
+  }
+  if constexpr (RAG && sizeof(T) == 4) {
+    zvz = dzm_rows4(a.Dz, [&](int q) { return q == 0 ? win4(hvz, 4) : lds4(s_vz + wb + q * BW + 4); });
+    zvx = dzp_rows4(a.Dz, [&](int q) { return q == 0 ? win4(hvx, 4) : lds4(s_vx + wb + q * BW + 4); });
   }
   if (AFDA && gj < L + 4) {  // on the surface row the tau_zz = 0 relation sets e_zz
     const int qs = gj - L;
@@ -191,7 +196,7 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
   {
     Q4<T> exx = splat4<T>(0), ezz = exx, exz = exx;
     if (act) {
-      tti_rates4<T, BW, AFDA>(a, s_vx, s_vz, (r + 5) * BW + lx + 4, gi0, gj, true, rxx, rzz, rxz);
+      tti_rates4<T, BW, AFDA, RAG>(a, s_vx, s_vz, (r + 5) * BW + lx + 4, gi0, gj, true, rxx, rzz, rxz);
       tti_effective4<T, NSLS>(tau, mxx, mzz, mxz, rxx, rzz, rxz, exx, ezz, exz);
       if (RAG && gi0 + 4 > xe) {  // zero outside U
         zero_edge4(exx, xe - gi0);
@@ -208,7 +213,7 @@ __device__ __forceinline__ void split_stress_tti_tile(const StepArgs<T> &a, cons
     Q4<T> exx = splat4<T>(0), ezz = exx, exz = exx;
     if (ract) {
       Q4<T> qxx, qzz, qxz;
-      tti_rates4<T, BW, AFDA>(a, s_vx, s_vz, (rr + 4) * BW + rc, rgi0, rgj, false, qxx, qzz, qxz);
+      tti_rates4<T, BW, AFDA, RAG>(a, s_vx, s_vz, (rr + 4) * BW + rc, rgi0, rgj, false, qxx, qzz, qxz);
       tti_effective4<T, NSLS>(rtau, qmxx, qmzz, qmxz, qxx, qzz, qxz, exx, ezz, exz);
       if (RAG && rgi0 + 4 > xe) {
         zero_edge4(exx, xe - rgi0);

@@ -327,6 +327,22 @@ __device__ __forceinline__ void zero_edge4(Q4<T> &q, int n) {
   for (int k = 0; k < 4; ++k)
     if (k >= n) q.v[k] = T(0);
 }
+// z derivatives of 4 cells from row(q), q rows below them, as differences of
+// pairs of rows
+template <typename T, typename F>
+__device__ __forceinline__ Q4<T> dzm_rows4(const T *D, F row) {
+  Q4<T> s = mul4(splat4<T>(D[0]), sub4(row(0), row(-1)));
+#pragma unroll
+  for (int q = 1; q < 4; ++q) s = fma4(splat4<T>(D[q]), sub4(row(q), row(-1 - q)), s);
+  return s;
+}
+template <typename T, typename F>
+__device__ __forceinline__ Q4<T> dzp_rows4(const T *D, F row) {
+  Q4<T> s = mul4(splat4<T>(D[0]), sub4(row(1), row(0)));
+#pragma unroll
+  for (int q = 1; q < 4; ++q) s = fma4(splat4<T>(D[q]), sub4(row(1 + q), row(-q)), s);
+  return s;
+}
 // window of 4 consecutive values of a 12-value row, starting at o
 template <typename T>
 __device__ __forceinline__ Q4<T> win4(const T (&u)[12], int o) {
