@@ -29,6 +29,7 @@
 // c55, tau) — for ISO c13 = lambda and c55 = mu carry dJ/dlambda and
 // dJ/dmu.  vi_gradient_velocity maps them to (vp, vs, rho, 1/Q) and, for
 // VTI, vi_gradient_thomsen to the Thomsen (epsilon, delta).
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 #include <vector>
@@ -834,27 +835,52 @@ __global__ void __launch_bounds__(AdjGeom<T>::NT, 5)
   pdl_release();
   if (!boxes_landed(bar, x.err)) return;
   const int ow = t.r * G::WX + t.lx + 4, oz = t.r * G::TX + t.lx;
-  if (e0 < e1) {  // a tile with entries: its residuals into the staged v adjoint, one thread per receiver
+  Pk<T> vx{}, vz{};
+  if (t.act) {
+    vx = psub(ldv(box(SM::VB) + oz),
+              padd(dxp(ldwin(box(SM::R0) + ow), A.Dx), dzm(box(SM::R2) + oz + 4 * G::TX, G::TX, A.Dz)));
+    vz = psub(ldv(box(SM::VB) + PL + oz),
+              padd(dzp(box(SM::R1) + oz + 3 * G::TX, G::TX, A.Dz), dxm(ldwin(box(SM::R3) + ow), A.Dx)));
+    if (t.gi0 + V > A.nx - L) {
+      zero_outside(vx, A.nx - L - t.gi0);
+      zero_outside(vz, A.nx - L - t.gi0);
+    }
+  }
+  if (e0 < e1) {  // a tile with entries: its residuals added in shared memory, one thread per receiver cell
     T *sv = box(SM::VB);
-    for (int e = e0 + (int)threadIdx.x; e < e1; e += G::NT) {
-      const int4 en = x.tile_ent[e];
-      if (en.w != TL_RECEIVER) continue;
-      const long long r = (long long)en.y * ld + en.x;
-      const int o = (en.y - t.z0) * G::TX + en.x - t.x0;
-      atomicAdd(sv + o, x1.vx()[r] - obs[(long long)en.z * x.tnt + x.it]);
-      atomicAdd(sv + PL + o, x1.vz()[r] - obs[(long long)(x.nrec + en.z) * x.tnt + x.it]);
+    if (t.act) {
+      stv(sv + oz, vx);
+      stv(sv + PL + oz, vz);
     }
     __syncthreads();
+    for (int e = e0 + (int)threadIdx.x; e < e1; e += G::NT) {
+      int4 en = x.tile_ent[e];
+      if (en.w != TL_RECEIVER) continue;
+      const int i = en.x, j = en.y;
+      if (e > e0) {  // receivers of a cell follow each other: its first one's thread takes them all
+        const int4 b = x.tile_ent[e - 1];
+        if (b.w == TL_RECEIVER && b.x == i && b.y == j) continue;
+      }
+      const T dx = x1.vx()[(long long)j * ld + i], dz = x1.vz()[(long long)j * ld + i];
+      const int o = (j - t.z0) * G::TX + i - t.x0;
+      T ax = sv[o], az = sv[PL + o];
+      int f = e;
+      do {
+        ax += dx - obs[(long long)en.z * x.tnt + x.it];
+        az += dz - obs[(long long)(x.nrec + en.z) * x.tnt + x.it];
+        if (++f == e1) break;
+        en = x.tile_ent[f];
+      } while (en.x == i && en.y == j);
+      sv[o] = ax;
+      sv[PL + o] = az;
+    }
+    __syncthreads();
+    if (t.act) {
+      vx = ldv(sv + oz);
+      vz = ldv(sv + PL + oz);
+    }
   }
   if (!t.act) return;
-  Pk<T> vx = psub(ldv(box(SM::VB) + oz),
-                  padd(dxp(ldwin(box(SM::R0) + ow), A.Dx), dzm(box(SM::R2) + oz + 4 * G::TX, G::TX, A.Dz)));
-  Pk<T> vz = psub(ldv(box(SM::VB) + PL + oz),
-                  padd(dzp(box(SM::R1) + oz + 3 * G::TX, G::TX, A.Dz), dxm(ldwin(box(SM::R3) + ow), A.Dx)));
-  if (t.gi0 + V > A.nx - L) {
-    zero_outside(vx, A.nx - L - t.gi0);
-    zero_outside(vz, A.nx - L - t.gi0);
-  }
   stv(vb + c, vx);
   stv(vb + np + c, vz);
   // forward stress divergence of the step
@@ -1493,6 +1519,12 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
     build_tile_lists(c.nx, c.nz, SG::TX, SG::TZ, 0, shot, off, ent, ntx, ntz);
     build_tile_lists(c.nx, c.nz, tti ? STG::TX : SS::TX, tti ? STG::TZ : SS::TZ, 0, shot, soff, sent, sntx, sntz);
     build_tile_lists(c.nx, c.nz, AG::TX, AG::TZ, 0, shot, aoff, aent, antx, antz);
+    // a tile's receivers by cell, in the order of the list within one (k_adj_vel)
+    for (size_t k = 0; k + 1 < aoff.size(); ++k)
+      std::stable_sort(aent.begin() + aoff[k], aent.begin() + aoff[k + 1], [](const int4 &u, const int4 &v) {
+        if (u.w != v.w || u.w != TL_RECEIVER) return u.w < v.w;
+        return u.y != v.y ? u.y < v.y : u.x < v.x;
+      });
     const int nvoff = (int)off.size();
     for (int v : soff) off.push_back(v + (int)ent.size());
     ent.insert(ent.end(), sent.begin(), sent.end());
