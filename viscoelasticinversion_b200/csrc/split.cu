@@ -488,8 +488,9 @@ int split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int nsteps
 // ---- grids whose rows the split kernels cannot take as they are ----------
 
 // Copies planes between row strides: columns [c0, c1), rows from r0 (planes
-// 2 .. 4: from r0s) to r1.  One plane per blockIdx.z, 8 rows x 128 columns
-// per block.  Bandwidth bound: each value read and written once.
+// 2 .. 4: from r0s) to r1.  One plane per blockIdx.y; 8 rows x 128 columns per
+// block, nxb blocks across (in one grid dimension: tall grids have more than
+// 65535 rows of blocks).  Bandwidth bound: each value read and written once.
 template <typename T>
 struct PadPlanes {
   const T *src[5 + 3 * VI_MAX_SLS + 8];
@@ -497,16 +498,22 @@ struct PadPlanes {
 };
 template <typename T>
 __global__ void __launch_bounds__(256) k_copy_planes(const __grid_constant__ PadPlanes<T> pl, int lds, int ldd, int c0,
-                                                     int c1, int r0, int r0s, int r1) {
-  const int q = blockIdx.z, j = blockIdx.y * 8 + threadIdx.x / 32;
+                                                     int c1, int r0, int r0s, int r1, int nxb) {
+  const int q = blockIdx.y, bx = (int)blockIdx.x % nxb, j = (int)blockIdx.x / nxb * 8 + (int)threadIdx.x / 32;
   if (j < (q >= 2 && q < 5 ? r0s : r0) || j >= r1) return;
   const T *src = pl.src[q] + (long long)j * lds;
   T *dst = pl.dst[q] + (long long)j * ldd;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int i = c0 + (int)blockIdx.x * 128 + 32 * k + (int)(threadIdx.x % 32);
+    const int i = c0 + bx * 128 + 32 * k + (int)(threadIdx.x % 32);
     if (i < c1) dst[i] = src[i];
   }
+}
+template <typename T>
+static void launch_copy_planes(const PadPlanes<T> &pl, int n, int lds, int ldd, int c0, int c1, int r0, int r0s, int r1,
+                               cudaStream_t st) {
+  const int nxb = (c1 - c0 + 127) / 128, nzb = (r1 + 7) / 8;
+  k_copy_planes<T><<<dim3(nxb * nzb, n), 256, 0, st>>>(pl, lds, ldd, c0, c1, r0, r0s, r1, nxb);
 }
 
 template <typename T>
@@ -516,7 +523,7 @@ int copy_planes(const T *const *src, T *const *dst, int n, int lds, int ldd, int
     pl.src[q] = src[q];
     pl.dst[q] = dst[q];
   }
-  k_copy_planes<T><<<dim3((nx + 127) / 128, (nz + 7) / 8, n), 256, 0, st>>>(pl, lds, ldd, 0, nx, 0, 0, nz);
+  launch_copy_planes(pl, n, lds, ldd, 0, nx, 0, 0, nz, st);
   return cuda_check(cudaGetLastError(), "copy planes launch");
 }
 template int copy_planes<float>(const float *const *, float *const *, int, int, int, int, int, cudaStream_t);
@@ -560,7 +567,7 @@ int padded_split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int
     }
   T *const user_m = a.m;
   const long long user_ms = a.mstride;
-  k_copy_planes<T><<<dim3((nx + 127) / 128, (nz + 7) / 8, q), 256, 0, st>>>(pl, nx, ld, 0, nx, 0, 0, nz);
+  launch_copy_planes(pl, q, nx, ld, 0, nx, 0, 0, nz, st);
   if ((rc = cuda_check(cudaGetLastError(), "pad launch"))) return rc;
   a.ld = ld;
   a.vx = base;
@@ -577,8 +584,7 @@ int padded_split_steps(vi_plan *p, StepArgs<T> a, const vi_shot *s, int it0, int
     pl.src[k] = k < 5 ? base + k * np : m_last + (k - 5) * np;
     pl.dst[k] = k < 5 ? user[k] : user_m + (k - 5) * user_ms;
   }
-  k_copy_planes<T><<<dim3((nx - 2 * L + 127) / 128, (nz + 7) / 8, ns), 256, 0, st>>>(pl, ld, nx, L, nx - L, L, 0,
-                                                                                     nz - L);
+  launch_copy_planes(pl, ns, ld, nx, L, nx - L, L, 0, nz - L, st);
   return cuda_check(cudaGetLastError(), "unpad launch");
 }
 
