@@ -37,6 +37,7 @@
 #include "fused.cuh"
 #include "nvtx.cuh"
 #include "fused_tma.cuh"
+#include "gradient.cuh"
 #include "pdl.cuh"
 #include "plan.cuh"
 #include "split.cuh"
@@ -1403,6 +1404,31 @@ __global__ void k_tti_param_grad(long long np, const double *g, const double *vp
 
 }  // namespace
 
+// Elements of the workspace: one state slot; rbar, dbar, TTI's effective rates,
+// the FP64 accumulators and the medium copies.
+template <typename T>
+static long long slot_elems(const vi_config &c) {
+  const long long ld = (c.nx + 3) / 4 * 4, Lp = c.pml_thickness;
+  const long long wx = Lp * ((c.pml_left ? 1 : 0) + (c.pml_right ? 1 : 0));
+  const long long hz = Lp * ((c.pml_top ? 1 : 0) + (c.pml_bottom ? 1 : 0));
+  return Slot<T>::size(ld * c.nz, wx * c.nz, ld * hz, c.nsls);
+}
+template <typename T>
+static long long scratch_elems(const vi_config &c, int copied) {
+  const long long np = (long long)((c.nx + 3) / 4 * 4) * c.nz, wide = sizeof(double) / sizeof(T);
+  return (8 + (c.medium == VI_MEDIUM_TTI ? 6 : 0) + acc_planes(c.medium) * wide + copied) * np;
+}
+template <typename T>
+static size_t gradient_bytes_t(const vi_config &c, long long nslots, int nt, int nrec, int copied) {
+  // (behind the traces: the misfit and its partial sums)
+  return sizeof(T) * (size_t)(nslots * slot_elems<T>(c) + scratch_elems<T>(c, copied) + 2LL * nrec * nt) + 64 +
+         8 * kMisfitBlocks;
+}
+size_t gradient_bytes(const vi_config &c, long long nslots, int nt, int nrec, int copied) {
+  return c.precision == VI_F64 ? gradient_bytes_t<double>(c, nslots, nt, nrec, copied)
+                               : gradient_bytes_t<float>(c, nslots, nt, nrec, copied);
+}
+
 template <typename T>
 static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, int nt, const T *obs,
                          int K, int accumulate, double *grad, double *misfit, cudaStream_t st) {
@@ -1421,7 +1447,7 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
   // same vector kernels
   const long long np = (long long)ld * c.nz;
   const long long px = (long long)p->wx * c.nz, pz = (long long)ld * p->hz;
-  const long long slot = Slot<T>::size(np, px, pz, N);
+  const long long slot = slot_elems<T>(c);
   const int nrec = shot->nrec;
   const long long ntr = 2LL * nrec * nt;
   // the medium where its planes are not laid out so already
@@ -1432,15 +1458,14 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
     copy_med |= ((uintptr_t)q & 15) != 0;
     nmed += q != nullptr;
   }
-  const long long wide = sizeof(double) / sizeof(T);
-  const long long scratch = (8 + (tti ? 6 : 0) + acc_planes(c.medium) * wide + (copy_med ? nmed : 0)) * np;
+  const int copied = copy_med ? nmed : 0;
   // K = 0: every state of the forward sweep kept in HBM when the sweep fits
   // in 60 % of the device's memory and in what is free (1024 x 512 x 3000
   // VTI FP32: 88 GB), so the adjoint reads each step's states and nothing
   // is recomputed; else checkpoints every ceil(sqrt(nt)) steps
   bool keep_all = false;
   if (K <= 0) {
-    const size_t all = sizeof(T) * ((size_t)(nt + 2) * slot + scratch + ntr) + 64;
+    const size_t all = gradient_bytes(c, nt + 2LL, nt, nrec, copied);
     if (p->device_bytes > 0 && all <= p->fwd_bytes) {
       // the workspace holds the sweep already: nothing to ask the driver
       // (cudaMemGetInfo took up to 10 ms of a 10 ms gradient)
@@ -1461,7 +1486,7 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
   // workspace: checkpoints (keep_all: every state) | segment (K + 1 slots; none when keep_all) |
   // adjoint slot | rbar, dbar (4 planes each) | TTI: forward effective rates (6 planes) | FP64
   // accumulators | medium copies | traces | misfit
-  const size_t need = sizeof(T) * ((size_t)(nck + (keep_all ? 0 : K + 1) + 1) * slot + scratch + ntr) + 64 + 8 * kMisfitBlocks;
+  const size_t need = gradient_bytes(c, nck + (keep_all ? 0 : K + 1) + 1LL, nt, nrec, copied);
   size_t have = p->fwd_bytes;
   if ((rc = ensure_buffer(p, &p->fwd, &have, need))) return rc;
   p->fwd_bytes = have;
@@ -1471,7 +1496,7 @@ static int gradient_impl(vi_plan *p, const vi_medium *m, const vi_shot *shot, in
   T *rbar = adj + slot, *dbar = rbar + 4 * np, *fe = dbar + 4 * np;
   double *acc = (double *)(fe + (tti ? 6 * np : 0));
   T *pmed = (T *)(acc + acc_planes(c.medium) * np);
-  T *tr = pmed + (copy_med ? nmed * np : 0);
+  T *tr = pmed + copied * np;
   auto mk = [&](T *b) { return Slot<T>{b, np, px, pz, N}; };
   if ((rc = stage_shot<T>(p, shot, st))) return rc;
   vi_medium mw = *m;

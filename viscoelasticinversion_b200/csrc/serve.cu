@@ -41,6 +41,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "gradient.cuh"
 #include "nvtx.cuh"
 #include "plan.cuh"
 
@@ -118,35 +119,33 @@ double remaining_work(const Req &q) {
   return cells * left * (r.kind == VI_REQ_GRADIENT ? 3.0 : 1.0) * (r.cfg.medium == VI_MEDIUM_TTI ? 2.0 : 1.0);
 }
 
-// Device bytes a request holds while resident (plan workspace included,
-// rounded up): medium, state, the second state or padded copy, CPML
-// strips, wavelets and traces; for a gradient the checkpoints and segment
-// slots, the adjoint state and scratch, observed traces and FP64 planes.
+// Device bytes a request holds while resident, rounded up: its own buffers
+// (admit_impl) and its plan's: CPML memory, profiles, lists, and the workspace of
+// its steps (TTI's second state, the padded copies of odd rows) or of its
+// gradient.
 int64_t footprint(const vi_request &r) {
   const vi_config &c = r.cfg;
-  const int64_t np = (int64_t)c.nx * c.nz, e = (int64_t)esize_of(c);
-  const int64_t ns = 5 + 3 * (int64_t)c.nsls;
+  const int64_t nx = c.nx, nz = c.nz, np = nx * nz, e = (int64_t)esize_of(c);
+  const int64_t ld = (nx + 3) / 4 * 4, ns = 5 + 3 * (int64_t)c.nsls;
   const int64_t pml = c.pml_thickness > 0 ? c.pml_thickness : 0;
-  const int64_t psi = 2 * 4 * (2 * pml * c.nz + c.nx * 2 * pml) * e;
-  const int64_t tr = 2 * (int64_t)r.nrec * r.nt * e;
-  const int64_t wav = (int64_t)r.nsrc * (r.wavelet_nt > 0 ? r.wavelet_nt : 0) * e;
-  int64_t b = (8 + 2 * ns + 6) * np * e + psi + 2 * tr + wav + (16 << 20);
-  // odd rows: the padded copies hold the state and the medium (within the
-  // planes above for ISO and VTI) and TTI's second memory-variable set
-  if (c.nx % 4 != 0 && c.medium == VI_MEDIUM_TTI) b += (2 + 3 * (int64_t)c.nsls) * np * e;
-  if (r.kind == VI_REQ_GRADIENT) {
-    int64_t K = 1;
-    while (K * K < r.nt) ++K;
-    const int64_t nck = (r.nt + K - 1) / K;
-    const int64_t slot = ns * np * e + psi / 2;
-    // adjoint scratch: rbar, dbar, TTI's effective rates, odd rows' medium copy
-    // and the FP64 accumulators; what the forward-only planes above leave over
-    // (second state copy, spare) counts towards it
-    const bool tti = c.medium == VI_MEDIUM_TTI;
-    const int64_t scratch = (8 + (tti ? 6 : 0) + (c.nx % 4 != 0 ? 8 : 0)) * np * e + (tti ? 11 : 7) * np * 8;
-    b += (nck + K + 2) * slot + std::max(13 * np * e, scratch - (2 * ns + 6) * np * e) + 8 * np * 8 + tr;
-  }
-  return b;
+  const int64_t tr = 2 * (int64_t)r.nrec * r.nt;
+  const int64_t wav = (int64_t)r.nsrc * (r.wavelet_nt > 0 ? r.wavelet_nt : 0);
+  const bool grad = r.kind == VI_REQ_GRADIENT, tti = c.medium == VI_MEDIUM_TTI;
+  int64_t b = ((8 + ns) * np + wav + tr) * e;  // medium, state, wavelets, traces
+  b += kPsiPlanes * (2 * pml * nz + nx * 2 * pml) * e + 6 * (nx + nz) * e + np / 16 + (16 << 20);
+  // the step's second state or padded copies of state, medium and TTI's other
+  // memory variables; compensated stresses' residues
+  int64_t step = 0;
+  if (tti) step = ns * np * e;
+  if (nx % 4 != 0) step = (ns + 8 + (tti ? 3 * c.nsls : 0)) * ld * nz * e;
+  if (c.precision == VI_F32C) step += 6 * np;
+  if (!grad) return b + std::max(step, (ns + 6) * np * e);
+  // checkpoints every ceil(sqrt(nt)) steps, a segment, the adjoint state; a plan
+  // that ran a forward request before keeps that one's workspace too
+  int64_t K = 1;
+  while (K * K < r.nt) ++K;
+  const int64_t nck = (r.nt + K - 1) / K;
+  return b + step + tr * e + 8 * np * 8 + (int64_t)gradient_bytes(c, nck + K + 2, r.nt, r.nrec, nx % 4 != 0 ? 8 : 0);
 }
 
 }  // namespace
