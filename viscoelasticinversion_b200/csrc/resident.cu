@@ -8,7 +8,7 @@
 // stresses and coefficients in its shared memory, memory variables in
 // registers.  After each pass it hands the four cells along its edges to its
 // neighbours through a shadow of the planes in which every 32-bit word travels
-// beside the number of the pass that wrote it, in one 8-byte store: a reader
+// beside the number of the pass that wrote it, in one 64-bit element: a reader
 // polls the words themselves, so an exchange is one store and one load through
 // the L2, without fences, flags or a grid barrier (flags and fences took 4 us a
 // pass).  One shadow per pass suffices: a CTA rewrites its velocity edges only
@@ -211,20 +211,26 @@ __device__ __forceinline__ void wadd_lane(Pw<T, W> &q, int k, T d) {
     if (i == k) q.v[i] = add_rn(q.v[i], d);
 }
 
-// Edge cells beside their pass number: (word, pass) pairs, each an 8-byte unit
-// of its own, written as they come and read 4 cells at a time.
+// Edge cells beside their pass number: (word, pass) pairs, each one 64-bit element
+// of a relaxed access, written as they come and read 4 cells at a time (the
+// flag-in-word scheme of NCCL's LL protocol).  PTX promises a 64-bit element
+// whole, alone or in a vector, so a pair with the right number holds that pass's
+// word; the order of elements does not matter.
 __device__ __forceinline__ void st_pair2(uint32_t *p, uint32_t a, uint32_t b, uint32_t n) {
-  asm volatile("st.volatile.global.v4.u32 [%0], {%1, %3, %2, %3};" ::"l"(p), "r"(a), "r"(b), "r"(n) : "memory");
+  asm volatile("{\n .reg .b64 u, v;\n mov.b64 u, {%1, %3};\n mov.b64 v, {%2, %3};\n"
+               " st.relaxed.gpu.global.v2.b64 [%0], {u, v};\n}" ::"l"(p), "r"(a), "r"(b), "r"(n) : "memory");
 }
 __device__ __forceinline__ bool ld_pair2(const uint32_t *p, uint32_t &a, uint32_t &b, uint32_t n) {
   uint32_t f, g;
-  asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a), "=r"(f), "=r"(b), "=r"(g) : "l"(p) : "memory");
+  asm volatile("{\n .reg .b64 u, v;\n ld.relaxed.gpu.global.v2.b64 {u, v}, [%4];\n mov.b64 {%0, %1}, u;\n"
+               " mov.b64 {%2, %3}, v;\n}" : "=r"(a), "=r"(f), "=r"(b), "=r"(g) : "l"(p) : "memory");
   return f == n && g == n;
 }
 template <int W>
 __device__ __forceinline__ void st_edge(uint32_t *p, const Pw<float, W> &q, uint32_t n) {
   if constexpr (W == 1) {
-    asm volatile("st.volatile.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(__float_as_uint(q.v[0])), "r"(n) : "memory");
+    asm volatile("{\n .reg .b64 u;\n mov.b64 u, {%1, %2};\n st.relaxed.gpu.global.b64 [%0], u;\n}" ::"l"(p),
+                 "r"(__float_as_uint(q.v[0])), "r"(n) : "memory");
   } else {
 #pragma unroll
     for (int k = 0; k < W; k += 2) st_pair2(p + 2 * k, __float_as_uint(q.v[k]), __float_as_uint(q.v[k + 1]), n);
