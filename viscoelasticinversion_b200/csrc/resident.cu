@@ -40,6 +40,7 @@ struct ResGeom {
   int txg, tz, px, pz, threads, width;
   size_t smem;
 };
+constexpr size_t kResMaxSmem = 226 * 1024;
 constexpr int kResCoef = 7;  // C11, C13, C33, C55h, tau, bx, bz
 constexpr int kResPsi = 8;   // 4 planes of x-strip memory, 4 of z
 
@@ -597,7 +598,7 @@ static bool res_geometry(const vi_config &c, int nsm, ResGeom &out) {
       const int width = cells <= res_max_threads<T>() ? 1 : 2;
       const int threads = (cells / width + 31) / 32 * 32;
       const size_t smem = res_smem<T>(txg, tz);
-      if (items > 2 * threads || smem > 226 * 1024) continue;
+      if (items > 2 * threads || smem > kResMaxSmem) continue;
       found = true;
       best = cost;
       out = ResGeom{txg, tz, px, used, threads, width, smem};
@@ -640,7 +641,9 @@ template <typename T, int KIND, int NSLS, int W>
 static int launch_resident_w(const StepArgs<T> &a, const FusedExtras<T> &x, const ResGeom &g, int it0, int nsteps,
                              uint32_t *shadow, uint32_t pass0, cudaStream_t st) {
   auto k = k_resident<T, KIND, NSLS, W>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);
+  // one value whatever the tiling: the limit is the kernel's, and another thread
+  // may launch it for another grid between this call and the launch
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResMaxSmem);
   if (e != cudaSuccess) return cuda_check(e, "resident step smem attribute");
   StepArgs<T> av = a;
   FusedExtras<T> xv = x;
