@@ -188,7 +188,9 @@ int vi_plan_last_kernel(const vi_plan *plan, int32_t *kernel);
  * (sciml_solver/CPML.jl:291-328).  `shot` may be NULL (no sources or
  * receivers).  kernel_variant: 0 = default (with nx % 4 == 0 and 16-byte
  * aligned planes the split pair, for small ISO/VTI grids and enough steps
- * as one resident kernel per call; other rows and planes of 2048 cells or
+ * as resident kernels of up to 128 steps that take every SM: work of other
+ * streams that does not fit beside them waits for one of them, about 1 ms,
+ * before each of its kernels; variant 5 asks for the pair; other rows and planes of 2048 cells or
  * more on padded copies that the plan allocates, copied in and out every
  * call; the fused kernel for smaller ones and when there is no memory for
  * the copies), 1 = plain
