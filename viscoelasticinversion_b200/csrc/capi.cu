@@ -446,18 +446,17 @@ template int launch_finite_check<float>(const void *, const void *, const void *
 template int launch_finite_check<double>(const void *, const void *, const void *, long long, int *, int,
                                          cudaStream_t);
 
-// Grids of more than one tile of the fused kernel (64 x 32 cells) whose rows
-// or planes the split kernels cannot take as they are run the split pair on
-// padded copies (split.cu:padded_split_steps); a grid within one tile keeps
-// the fused kernel, one launch of one CTA per step.  Measured on B200, us per
-// step of a 64-step call, copies included, against the fused kernel: 47 x 45
-// ISO FP32 9.6 vs 33.5, 301 x 203 10.5 vs 35.8, 1001 x 501 VTI 18.6 vs 44.5
-// (FP64 38.7 vs 102, TTI 23.7 vs 52.8), 1403 x 597 VTI 24.6 vs 57.2; of a
-// 1-step call 1001 x 501 137 vs 196 (both then copy the whole state), 47 x 45
-// 59 vs 91.  The line is not a crossover (no size was found where the fused
-// kernel wins): tiny grids keep the path callers see reported for them.  The
-// choice depends on the grid alone, so steps divided over calls give the same
-// bits.
+// Rows and planes that the split kernels cannot take as they are: from this many
+// cells on the split pair on padded copies (split.cu:padded_split_steps), below it
+// the fused kernel.  Measured on B200, us per step of a 64-step call, copies
+// included, against the fused kernel: 47 x 45 ISO FP32 9.6 vs 33.5, 301 x 203 10.5
+// vs 35.8, 1001 x 501 VTI 18.6 vs 44.5 (FP64 38.7 vs 102, TTI 23.7 vs 52.8), 1403 x
+// 597 VTI 24.6 vs 57.2; of a 1-step call 1001 x 501 137 vs 196 (both then copy the
+// whole state), 47 x 45 59 vs 91.  The line is not a crossover (no size was found
+// where the fused kernel wins): grids below it keep the path callers see reported
+// for them.  The choice depends on the grid alone, so steps divided over calls give
+// the same bits, unless some of the calls find no memory for the copies: those run
+// the fused kernel, which rounds in another order.
 constexpr long long kPadMinCells = 2048;
 
 template <typename T>
@@ -541,7 +540,10 @@ static int step_impl(vi_plan *p, const vi_medium *m, vi_fields *f, const vi_shot
     p->last_kernel = variant == 0 ? 5 : variant;
   } else {
     rc = VI_ERR_BUDGET;
-    if (variant == 0 && (long long)p->cfg.nx * p->cfg.nz >= kPadMinCells)
+    // (a surface above fewer than 5 updated rows is left to the fused kernel, which
+    // refuses it)
+    const bool short_grid = p->cfg.free_surface && p->cfg.nz - 2 * L < L + 1;
+    if (variant == 0 && (long long)p->cfg.nx * p->cfg.nz >= kPadMinCells && !short_grid)
       rc = padded_split_steps<T>(p, a, s, it0, nsteps, st);
     p->last_kernel = 5;
     if (rc == VI_ERR_BUDGET) {  // small grids, or no memory for the padded planes
