@@ -190,10 +190,11 @@ int vi_plan_last_kernel(const vi_plan *plan, int32_t *kernel);
  * aligned planes the split pair, for small ISO/VTI grids and enough steps
  * as resident kernels of up to 128 steps that take every SM: work of other
  * streams that does not fit beside them waits for one of them, about 1 ms,
- * before each of its kernels; variant 5 asks for the pair; other rows and planes of 2048 cells or
- * more on padded copies that the plan allocates, copied in and out every
- * call; the fused kernel for smaller ones and when there is no memory for
- * the copies), 1 = plain
+ * before each of its kernels; variant 5 is always the pair; other rows and
+ * planes of 2048 cells or more on padded copies of state and medium that
+ * the plan allocates and keeps (up to 31 planes at 3 mechanisms), copied in
+ * and out every call; the fused kernel for smaller ones and when there is
+ * no memory for the copies), 1 = plain
  * multi-kernel path (in place), 2 = fused kernel without TMA, 3 = TMA-staged
  * fused kernel (persistent, two stages when they fit), 4 = TMA-staged fused
  * kernel with one stage, 5 = split velocity/stress kernel pair (one tile

@@ -267,8 +267,11 @@ struct HaloItem {
   int sv, ss;
 };
 
+// 64 registers a thread in FP32, 128 in FP64, also for blocks with fewer threads:
+// at 3 mechanisms (VTI) the time loop spills 180 bytes a thread with two cells in
+// FP32, 36 with one, and 76 with two in FP64.
 template <typename T>
-constexpr int res_max_threads() {  // 64 registers a thread in FP32, 128 in FP64
+constexpr int res_max_threads() {
   return sizeof(T) == 4 ? 1024 : 512;
 }
 
