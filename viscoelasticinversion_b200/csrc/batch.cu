@@ -614,6 +614,7 @@ extern "C" int vi_batch_create(const vi_config *cfgs, int32_t nshots, vi_batch *
 
 extern "C" int vi_batch_destroy(vi_batch *b) {
   if (!b) return VI_OK;
+  const CaptureAside aside;
   if (b->graph) cudaGraphExecDestroy(b->graph);
   if (b->dev) cudaFree(b->dev);
   if (b->err) cudaFree(b->err);

@@ -660,6 +660,7 @@ extern "C" int vi_plan_set_wave(vi_plan *p, int32_t depth, int32_t lag) {
 
 extern "C" int vi_plan_destroy(vi_plan *p) {
   if (!p) return VI_OK;
+  const CaptureAside aside;
   int prev = 0;
   cudaGetDevice(&prev);
   cudaSetDevice(p->device);

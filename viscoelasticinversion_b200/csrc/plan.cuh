@@ -89,6 +89,16 @@ void mark_steps(vi_plan *p, cudaStream_t st);
 // replayed; list staging refuses it whether or not it has something to copy.
 bool capturing(cudaStream_t st);
 int refuse_capture(cudaStream_t st);
+// While it lives, calls of this thread that a stream capture forbids (frees) do not
+// end a capture in progress: objects are destroyed whenever their owner drops them,
+// a garbage collector's run in the middle of a capture included.
+struct CaptureAside {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CaptureAside() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~CaptureAside() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  CaptureAside(const CaptureAside &) = delete;
+  CaptureAside &operator=(const CaptureAside &) = delete;
+};
 void mark_call(vi_plan *p, bool running);
 int cuda_check(cudaError_t e, const char *what);
 // Grow-only device buffer.
