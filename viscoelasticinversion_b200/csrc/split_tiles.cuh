@@ -148,8 +148,14 @@ __device__ __forceinline__ void split_vel_tile(const StepArgs<T> &a, const Fused
     }
   }
   if constexpr (RAG && sizeof(T) == 4) {
-    zxz = dzm_rows4(a.Dz, [&](int q) { return q == 0 ? win4(hxz, 4) : ldg4(a.sxz + g + (long long)q * ld); });
-    zzz = dzp_rows4(a.Dz, [&](int q) { return ldg4(a.szz + g + (long long)q * ld); });
+    const T *const qz = a.sxz + g, *const pz = a.szz + g;
+    zxz = mul4(splat4<T>(a.Dz[0]), sub4(win4(hxz, 4), ldg4(qz - ld)));
+    zzz = mul4(splat4<T>(a.Dz[0]), sub4(ldg4(pz + ld), ldg4(pz)));
+#pragma unroll
+    for (int q = 1; q < 4; ++q) {
+      zxz = fma4(splat4<T>(a.Dz[q]), sub4(ldg4(qz + (long long)q * ld), ldg4(qz - (q + 1LL) * ld)), zxz);
+      zzz = fma4(splat4<T>(a.Dz[q]), sub4(ldg4(pz + (q + 1LL) * ld), ldg4(pz - (long long)q * ld)), zzz);
+    }
   }
   if (AFDA && gj < L + 4) {  // one-sided z derivatives below the H-AFDA surface
     const int qs = gj - L;
