@@ -188,7 +188,7 @@ int vi_plan_last_kernel(const vi_plan *plan, int32_t *kernel);
  * (sciml_solver/CPML.jl:291-328).  `shot` may be NULL (no sources or
  * receivers).  kernel_variant: 0 = default (with nx % 4 == 0 and 16-byte
  * aligned planes the split pair, for small ISO/VTI grids and enough steps
- * as resident kernels of up to 128 steps that take every SM: work of other
+ * as resident kernels of up to 256 steps that take every SM: work of other
  * streams that does not fit beside them waits for one of them, about 1 ms,
  * before each of its kernels; variant 5 is always the pair; other rows and
  * planes of 2048 cells or more on padded copies of state and medium that

@@ -1,4 +1,4 @@
-// resident.cu — the split pair's time loop as one kernel per 128 steps, for ISO and
+// resident.cu — the split pair's time loop in kernels of many steps, for ISO and
 // VTI grids whose state fits on the chip.
 //
 // A small grid's step is all latency: two dependent launches of 3.6 us each
@@ -659,18 +659,19 @@ static int launch_resident_w(const StepArgs<T> &a, const FusedExtras<T> &x, cons
   }
   return cuda_check(e, "resident step launch");
 }
-// A call runs as launches of at most this many steps, so that a kernel of another
-// stream that does not fit beside the resident CTAs waits for one launch, not for
-// the call: a 4096^3 BF16 product issued after 3000 steps of 512 x 512 took 21.8
-// ms with one launch, 0.4 with 128 steps each, 0.37 with 64, 1.4 with 256 (0.16
-// beside the pair).  Another launch costs the state's way out and in: 3000 steps
-// of 512 x 512 22.73 -> 22.94 ms (64: 23.30), 256 x 256 10.74 -> 10.89, 512 x 256
-// FP64 19.21 -> 19.53 (64: 19.81).
-constexpr int kResidentLaunchSteps = 128;
+// A call runs as launches of at most this many steps, about a millisecond, so that
+// a kernel of another stream that does not fit beside the resident CTAs waits for
+// one launch, not for the call: a 4096^3 BF16 product issued after 3000 steps of
+// 512 x 512 took 21.8 ms with one launch, 0.4 with 128 steps each, 0.37 with 64,
+// 1.4 with 256 (0.16 beside the pair); of 256 x 256 10.3, 0.31, 0.23 and 0.36 ms.
+// Another launch costs the state's way out and in: 3000 steps of 512 x 512 22.73
+// -> 22.94 ms (64: 23.30), 256 x 256 10.74 -> 10.80 with 256 steps each (128:
+// 10.89, 64: 11.06).  Tilings with one cell a thread take half as long a step.
+constexpr int res_launch_steps(int width) { return width == 1 ? 256 : 128; }
 template <typename T, int KIND, int NSLS>
 static int launch_resident(const StepArgs<T> &a, const FusedExtras<T> &x, const ResGeom &g, int it0, int nsteps,
                            uint32_t *shadow, uint32_t pass0, cudaStream_t st) {
-  const int launches = (nsteps + kResidentLaunchSteps - 1) / kResidentLaunchSteps;
+  const int most = res_launch_steps(g.width), launches = nsteps / most + (nsteps % most != 0);
   for (int k = 0, done = 0; k < launches; ++k) {
     const int n = (nsteps - done) / (launches - k);  // even shares
     const uint32_t pass = pass0 + 2u * (uint32_t)done;
